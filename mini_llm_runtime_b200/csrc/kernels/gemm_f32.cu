@@ -6,78 +6,244 @@
 // Every output element is one accumulator that adds its K products in the order
 // k = 0, 1, ..., K-1 with fused multiply-adds.  The value of C[m,n] therefore depends
 // only on row m of A and row n of W, not on M, on the tile the element falls in, or on
-// what else is in the batch: the same token gives the same bits however the work is cut.
+// what else is in the batch: the same token gives the same bits however the work is cut,
+// and both kernels below give the same bits.
+//
+// Measured (one product, W from memory; before: one kernel of 64 x 64 tiles that waited for every 16 values of K):
+//   2 x 1024 x 3072 (M, N, K): 243 -> 20 us, bound by one thread's chain of multiply-adds; 2 x 151936 x 1024: 574 -> 100 us, 6.2 TB/s;
+//   129 x 1024 x 3072: 225 -> 55 us and 129 x 4096 x 1024: 164 -> 46 us, a few warps an SM, bound by their reads of shared memory;
+//   2048 x 4096 x 4096: 1970 -> 1663 us, 41 TFLOP/s, bound by shared memory.
+// Both stage rows of A and W as they lie in memory (asynchronous copies, several stages of K in
+// flight) with their stride padded by 16 bytes, so that 8 neighbouring rows read 4 values of K
+// each from different banks.
 #include "common.cuh"
 
 namespace {
 
-constexpr int BM = 64, BN = 64, BK = 16, TM = 4, TN = 4;
-
+// 16 bytes at column k of a row of K values, zeros past its end.
 template <bool kVector>
-__global__ void __launch_bounds__(256) gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W,
-                                                       float* __restrict__ C, int M, int N, int K, int lda,
-                                                       int ldw, int ldc) {
-    mlr_grid_dependents_may_start();
-    mlr_grid_wait();
-    __shared__ float As[BK][BM + 4];
-    __shared__ float Ws[BK][BN + 4];
-    const int tid = threadIdx.x;
-    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-    const int load_row = tid >> 2, load_k = (tid & 3) * 4;
-    const int tm = (tid >> 4) * TM, tn = (tid & 15) * TN;
-    float acc[TM][TN] = {};
-    for (int k0 = 0; k0 < K; k0 += BK) {
-        float a[4] = {0.f, 0.f, 0.f, 0.f}, w[4] = {0.f, 0.f, 0.f, 0.f};
-        const int k = k0 + load_k;
-        if (m0 + load_row < M) {
-            const float* src = A + static_cast<size_t>(m0 + load_row) * lda + k;
-            if (kVector && k + 3 < K) {
-                const float4 v = *reinterpret_cast<const float4*>(src);
-                a[0] = v.x; a[1] = v.y; a[2] = v.z; a[3] = v.w;
-            } else {
-#pragma unroll
-                for (int i = 0; i < 4; ++i) if (k + i < K) a[i] = src[i];
-            }
-        }
-        if (n0 + load_row < N) {
-            const float* src = W + static_cast<size_t>(n0 + load_row) * ldw + k;
-            if (kVector && k + 3 < K) {
-                const float4 v = *reinterpret_cast<const float4*>(src);
-                w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
-            } else {
-#pragma unroll
-                for (int i = 0; i < 4; ++i) if (k + i < K) w[i] = src[i];
-            }
-        }
-        __syncthreads();
+__device__ __forceinline__ void stage4(float* dst, const float* row, int k, int K, bool real) {
+    const unsigned to = static_cast<unsigned>(__cvta_generic_to_shared(dst));
+    if (kVector) {
+        const int bytes = real ? max(0, min(16, (K - k) * 4)) : 0;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(to), "l"(bytes ? row + k : row), "r"(bytes) : "memory");
+    } else {
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            As[load_k + i][load_row] = a[i];
-            Ws[load_k + i][load_row] = w[i];
-        }
-        __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < BK; ++kk) {
-            const float4 av = *reinterpret_cast<const float4*>(&As[kk][tm]);
-            const float4 wv = *reinterpret_cast<const float4*>(&Ws[kk][tn]);
-            const float ar[TM] = {av.x, av.y, av.z, av.w};
-            const float wr[TN] = {wv.x, wv.y, wv.z, wv.w};
-#pragma unroll
-            for (int i = 0; i < TM; ++i)
-#pragma unroll
-                for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(ar[i], wr[j], acc[i][j]);
+            const int bytes = real && k + i < K ? 4 : 0;
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(to + 4 * i), "l"(bytes ? row + k + i : row), "r"(bytes) : "memory");
         }
     }
+}
+template <int N>
+__device__ __forceinline__ void stages_left() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
+
+// ---- a tile of BM x BN outputs a block, TM x TN of them a thread (rows and columns dealt round the block) ----
+// Shared memory hands a warp 32 registers a cycle, however few addresses they come from, and the SM's schedulers issue four
+// multiply-adds a warp in that cycle: a thread's TM + TN values of a k for TM * TN multiply-adds bind all tiles but the largest.
+template <int BM, int BN, int TM, int TN, int STAGES, int KK = 32>
+struct Tile {
+    static constexpr int kRows = BM, kColumns = BN, kThreadRows = TM, kThreadColumns = TN;
+    static constexpr int kThreads = (BM / TM) * (BN / TN);
+    static constexpr int kStages = STAGES, kK = KK, kLd = kK + 4;
+    static constexpr size_t kShared = sizeof(float) * kStages * (BM + BN) * kLd;
+};
+
+template <bool kVector, typename T>
+__global__ void __launch_bounds__(T::kThreads) gemm_f32_tile_kernel(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw,
+                                                                    int ldc) {
+    constexpr int BM = T::kRows, BN = T::kColumns, TM = T::kThreadRows, TN = T::kThreadColumns;
+    extern __shared__ __align__(16) float staged[];           // per stage: A [BM][kLd], W [BN][kLd]
+    constexpr int kAcross = BN / TN, kDown = BM / TM, kStage = (BM + BN) * T::kLd, kChunks = T::kK / 4;
+    const int tid = threadIdx.x, tx = tid % kAcross, ty = tid / kAcross;
+    // Neighbouring blocks share W's rows, so that they come from memory once.
+    const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
+    const int steps = (K + T::kK - 1) / T::kK;
+    auto fetch_a = [&](int step) {
+        float* to = staged + (step % T::kStages) * kStage;
+#pragma unroll
+        for (int i = tid; i < BM * kChunks; i += T::kThreads) {
+            const int r = i / kChunks, c = (i % kChunks) * 4;
+            stage4<kVector>(to + r * T::kLd + c, m0 + r < M ? A + static_cast<size_t>(m0 + r) * lda : A, step * T::kK + c, K, m0 + r < M);
+        }
+    };
+    auto fetch_w = [&](int step) {
+        float* to = staged + (step % T::kStages) * kStage + BM * T::kLd;
+#pragma unroll
+        for (int i = tid; i < BN * kChunks; i += T::kThreads) {
+            const int r = i / kChunks, c = (i % kChunks) * 4;
+            stage4<kVector>(to + r * T::kLd + c, n0 + r < N ? W + static_cast<size_t>(n0 + r) * ldw : W, step * T::kK + c, K, n0 + r < N);
+        }
+    };
+    mlr_grid_wait();
+    for (int step = 0; step < T::kStages - 1; ++step) {
+        if (step < steps) { fetch_w(step); fetch_a(step); }
+        mlr_async_commit();
+    }
+    float acc[TM][TN] = {};
+    for (int step = 0; step < steps; ++step) {
+        stages_left<T::kStages - 2>();
+        __syncthreads();           // this step's stage has landed for everyone, and everyone is done with the one refilled next
+        if (step + T::kStages - 1 < steps) { fetch_w(step + T::kStages - 1); fetch_a(step + T::kStages - 1); }
+        mlr_async_commit();
+        const float* as = staged + (step % T::kStages) * kStage + ty * T::kLd;
+        const float* ws = staged + (step % T::kStages) * kStage + (BM + tx) * T::kLd;
+#pragma unroll
+        for (int kk = 0; kk < T::kK; kk += 4) {
+            float a[TM][4], w[TN][4];
+#pragma unroll
+            for (int i = 0; i < TM; ++i) mlr_load4(as + i * kDown * T::kLd + kk, a[i]);
+#pragma unroll
+            for (int j = 0; j < TN; ++j) mlr_load4(ws + j * kAcross * T::kLd + kk, w[j]);
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+#pragma unroll
+                for (int i = 0; i < TM; ++i)
+#pragma unroll
+                    for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i][q], w[j][q], acc[i][j]);
+        }
+    }
+    mlr_grid_dependents_may_start();
 #pragma unroll
     for (int i = 0; i < TM; ++i) {
-        const int m = m0 + tm + i;
+        const int m = m0 + ty + i * kDown;
         if (m >= M) continue;
 #pragma unroll
         for (int j = 0; j < TN; ++j) {
-            const int n = n0 + tn + j;
+            const int n = n0 + tx + j * kAcross;
             if (n < N) C[static_cast<size_t>(m) * ldc + n] = acc[i][j];
         }
     }
+}
+
+// ---- up to four rows (a decode step): a pass over W.  A block takes BN rows of W; thread (n, g) has row n of them and the rows g, g + G,
+// .. of A, G = 128 / BN.  W's first stages are on their way before the kernel before this one has ended (no kernel writes weights).
+constexpr int kFewRows = 4, kFewThreads = 128, kFewK = 64, kFewLd = kFewK + 4;
+constexpr size_t few_shared(int bn, int stages, int rows) { return sizeof(float) * stages * (bn + rows) * kFewLd; }
+
+template <bool kVector, int BN, int STAGES, int MT>
+__global__ void __launch_bounds__(kFewThreads) gemm_f32_few_kernel(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw,
+                                                                   int ldc) {
+    extern __shared__ __align__(16) float staged[];           // per stage: W [BN][kFewLd], A [M][kFewLd]
+    constexpr int kGroups = kFewThreads / BN, kChunks = kFewK / 4;
+    const int tid = threadIdx.x, n = tid % BN, g = tid / BN;
+    const int n0 = blockIdx.x * BN, stage_floats = (BN + M) * kFewLd;
+    const int steps = (K + kFewK - 1) / kFewK;
+    auto fetch_w = [&](int step) {
+        float* to = staged + (step % STAGES) * stage_floats;
+#pragma unroll
+        for (int i = tid; i < BN * kChunks; i += kFewThreads) {
+            const int r = i / kChunks, c = (i % kChunks) * 4;
+            stage4<kVector>(to + r * kFewLd + c, n0 + r < N ? W + static_cast<size_t>(n0 + r) * ldw : W, step * kFewK + c, K, n0 + r < N);
+        }
+    };
+    auto fetch_a = [&](int step) {
+        float* to = staged + (step % STAGES) * stage_floats + BN * kFewLd;
+        for (int i = tid; i < M * kChunks; i += kFewThreads) {
+            const int r = i / kChunks, c = (i % kChunks) * 4;
+            stage4<kVector>(to + r * kFewLd + c, A + static_cast<size_t>(r) * lda, step * kFewK + c, K, true);
+        }
+    };
+    for (int step = 0; step < STAGES - 1 && step < steps; ++step) fetch_w(step);
+    mlr_grid_wait();
+    // The first group to complete holds all of W's first stages and A's first; the later ones A's alone.
+    for (int step = 0; step < STAGES - 1; ++step) {
+        if (step < steps) fetch_a(step);
+        mlr_async_commit();
+    }
+    float acc[MT] = {};
+    for (int step = 0; step < steps; ++step) {
+        stages_left<STAGES - 2>();
+        __syncthreads();
+        if (step + STAGES - 1 < steps) { fetch_w(step + STAGES - 1); fetch_a(step + STAGES - 1); }
+        mlr_async_commit();
+        if ((tid & ~31) / BN >= M) continue;          // none of this warp's threads has a row of A (it still fetches for the others)
+        const float* ws = staged + (step % STAGES) * stage_floats + n * kFewLd;
+        const float* as = staged + (step % STAGES) * stage_floats + BN * kFewLd;
+#pragma unroll 8
+        for (int kk = 0; kk < kFewK; kk += 4) {
+            float w[4];
+            mlr_load4(ws + kk, w);
+#pragma unroll
+            for (int i = 0; i < MT; ++i) {
+                float a[4];
+                mlr_load4(as + min(g + i * kGroups, M - 1) * kFewLd + kk, a);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) acc[i] = fmaf(a[q], w[q], acc[i]);
+            }
+        }
+    }
+    mlr_grid_dependents_may_start();
+#pragma unroll
+    for (int i = 0; i < MT; ++i) {
+        const int m = g + i * kGroups;
+        if (m < M && n0 + n < N) C[static_cast<size_t>(m) * ldc + n0 + n] = acc[i];
+    }
+}
+
+template <typename Kernel>
+int allow_shared(Kernel kernel, size_t bytes) {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
+    return e == cudaSuccess ? 0 : mlr_fail("gemm_f32: cannot use %zu bytes of shared memory: %s", bytes, cudaGetErrorString(e));
+}
+
+struct Product {
+    const float *A, *W;
+    float* C;
+    int M, N, K, lda, ldw, ldc;
+    cudaStream_t stream;
+};
+
+template <bool kVector, typename T>
+int launch_tile(const Product& p) {
+    const dim3 grid((p.M + T::kRows - 1) / T::kRows, (p.N + T::kColumns - 1) / T::kColumns);
+    MLR_REQUIRE(grid.y <= 65535, "gemm_f32: N=%d needs more than 65535 column tiles", p.N);
+    if (allow_shared(gemm_f32_tile_kernel<kVector, T>, T::kShared)) return 1;
+    mlr_launch((gemm_f32_tile_kernel<kVector, T>), grid, dim3(T::kThreads), T::kShared, p.stream, p.A, p.W, p.C, p.M, p.N, p.K, p.lda, p.ldw, p.ldc);
+    return 0;
+}
+
+template <bool kVector, int BN, int STAGES, int MT>
+int launch_few(const Product& p) {
+    if (allow_shared(gemm_f32_few_kernel<kVector, BN, STAGES, MT>, few_shared(BN, STAGES, kFewRows))) return 1;
+    mlr_launch((gemm_f32_few_kernel<kVector, BN, STAGES, MT>), dim3((p.N + BN - 1) / BN), dim3(kFewThreads), few_shared(BN, STAGES, p.M), p.stream, p.A, p.W,
+               p.C, p.M, p.N, p.K, p.lda, p.ldw, p.ldc);
+    return 0;
+}
+
+// What a tile costs a value of K, in cycles of the busiest SM: the registers its warps read from shared memory (1.4 cycles each as
+// measured), or, with few warps, one warp's own way through reads, multiply-adds and its share of the staging.  The constants fit
+// what the tiles measured at 129 rows (6 x 8 a thread: 86 cycles where 78 are computed, 6 x 4: 47 and 48, 4 x 4 in two warps: 57 and 40).
+template <typename T>
+double tile_cost(int M, int N) {
+    const long long blocks = ((M + T::kRows - 1LL) / T::kRows) * ((N + T::kColumns - 1LL) / T::kColumns);
+    const double warps = static_cast<double>((blocks + mlr_sm_count() - 1) / mlr_sm_count()) * (T::kThreads / 32);
+    const double reads = 1.4 * warps * (T::kThreadRows + T::kThreadColumns);
+    const double alone = 10.0 + T::kThreadRows + T::kThreadColumns + T::kThreadRows * T::kThreadColumns + 3.0 * (T::kRows + T::kColumns) / T::kThreads;
+    return reads > alone ? reads : alone;
+}
+
+template <bool kVector, typename... Tiles>
+int launch_cheapest(const Product& p) {
+    const double costs[] = {tile_cost<Tiles>(p.M, p.N)...};
+    int (*const launches[])(const Product&) = {launch_tile<kVector, Tiles>...};
+    int best = 0;
+    for (int i = 1; i < static_cast<int>(sizeof...(Tiles)); ++i)
+        if (costs[i] < costs[best]) best = i;
+    return launches[best](p);
+}
+
+template <bool kVector>
+int choose(const Product& p) {
+    if (p.M <= kFewRows) {
+        // Wide blocks where they still give every SM two; with narrow ones a thread's chain of K multiply-adds is the bound, and
+        // sixteen stages hold most of its K in flight.
+        if (p.N >= 64 * 2 * mlr_sm_count()) return p.M <= 2 ? launch_few<kVector, 64, 4, 1>(p) : launch_few<kVector, 64, 4, 2>(p);
+        if (p.N >= 16 * 2 * mlr_sm_count()) return launch_few<kVector, 16, 16, 1>(p);
+        return launch_few<kVector, 8, 16, 1>(p);
+    }
+    return launch_cheapest<kVector, Tile<64, 128, 8, 8, 3>, Tile<48, 128, 6, 8, 3>, Tile<32, 128, 4, 8, 3>, Tile<48, 32, 3, 4, 4, 64>,
+                           Tile<16, 64, 2, 4, 4, 64>, Tile<16, 128, 8, 4, 4>, Tile<8, 128, 4, 4, 4>, Tile<16, 32, 2, 2, 5, 64>, Tile<8, 32, 1, 2, 5, 64>>(p);
 }
 
 }  // namespace
@@ -87,13 +253,9 @@ MLR_API int mlr_gemm_f32(const float* A, const float* W, float* C, int M, int N,
     MLR_REQUIRE(M >= 0 && N > 0 && K > 0, "gemm_f32: bad sizes M=%d N=%d K=%d", M, N, K);
     MLR_REQUIRE(lda >= K && ldw >= K && ldc >= N, "gemm_f32: a leading dimension is smaller than its row");
     if (M == 0) return 0;
-    const dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
-    MLR_REQUIRE(grid.y <= 65535, "gemm_f32: M=%d needs more than 65535 row tiles", M);
     const bool vector = lda % 4 == 0 && ldw % 4 == 0 && reinterpret_cast<uintptr_t>(A) % 16 == 0 &&
                         reinterpret_cast<uintptr_t>(W) % 16 == 0;
-    if (vector)
-        mlr_launch((gemm_f32_kernel<true>), dim3(grid), dim3(256), 0, stream, A, W, C, M, N, K, lda, ldw, ldc);
-    else
-        mlr_launch((gemm_f32_kernel<false>), dim3(grid), dim3(256), 0, stream, A, W, C, M, N, K, lda, ldw, ldc);
+    const Product p = {A, W, C, M, N, K, lda, ldw, ldc, stream};
+    if (vector ? choose<true>(p) : choose<false>(p)) return 1;
     return mlr_launched("gemm_f32");
 }

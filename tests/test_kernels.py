@@ -161,6 +161,25 @@ def test_gemm_f32_is_true_float32_and_independent_of_batching(M, N, K):
     assert torch.equal(out2, out)
 
 
+@pytest.mark.parametrize("M,N,K,aligned", [(2, 19000, 72, True), (4, 18945, 65, True), (4, 5000, 1100, True), (3, 129, 3072, False), (5, 31, 64, True),
+                                           (8, 4096, 96, True), (16, 130, 200, True), (17, 257, 33, False), (33, 2048, 64, True), (49, 6144, 40, True),
+                                           (129, 1024, 68, True), (129, 4099, 31, False), (200, 9000, 36, True), (1025, 2050, 36, True)])
+def test_gemm_f32_every_tile_gives_the_bits_of_a_row_alone(M, N, K, aligned):
+    """Sizes on both sides of the lines between the kernels and their tiles, operands on 16-byte borders and off them: every row has the
+    bits that the row has alone, and the sums are right."""
+    off = 0 if aligned else 1
+    a = torch.randn(M, K + 8, generator=gen(2)).to(DEV)[:, off:off + K]
+    w = torch.randn(N, K + 8, generator=gen(3)).to(DEV)[:, off:off + K]
+    out = torch.full((M, N), float("nan"), device=DEV)
+    F().gemm_f32(a, w, out)
+    bound = 2e-7 * math.sqrt(K) * (a.abs().double() @ w.abs().double().T) + 1e-6       # as above
+    assert ((out.double() - a.double() @ w.double().T).abs() <= bound).all()
+    for row in sorted({0, M // 2, M - 1}):
+        alone = torch.empty(1, N, device=DEV)
+        F().gemm_f32(a[row:row + 1], w, alone)
+        assert torch.equal(alone[0], out[row]), row
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 64, 64), (8, 4096, 4096), (3, 100, 96), (16, 515, 1056), (64, 300, 200), (65, 256, 64),
                                    (128, 256, 4096), (200, 515, 136), (2048, 6144, 4096), (300, 48, 12288), (129, 24, 72)])
 @pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])

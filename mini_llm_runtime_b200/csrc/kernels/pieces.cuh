@@ -72,6 +72,53 @@ __device__ __forceinline__ float4 piece_sum(const Pieces& p, const StagedPieces&
     return v;
 }
 
+// The same for NQ groups of four columns of a row, i + k * step (k = 0 .. NQ - 1, those below `width`): a piece's loads are on
+// their way together, the order of every sum is that of `piece_sum`.
+template <int NQ>
+__device__ __forceinline__ void piece_sums(const Pieces& p, const StagedPieces& s, int row, int i, int step, int width, float4 (&v)[NQ]) {
+    const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    auto add = [&](float w, const float4 (&e)[NQ]) {
+#pragma unroll
+        for (int k = 0; k < NQ; ++k) {
+            v[k].x = fmaf(w, e[k].x, v[k].x); v[k].y = fmaf(w, e[k].y, v[k].y);
+            v[k].z = fmaf(w, e[k].z, v[k].z); v[k].w = fmaf(w, e[k].w, v[k].w);
+        }
+    };
+#pragma unroll
+    for (int k = 0; k < NQ; ++k) v[k] = zero;
+    float4 shared[NQ], passed[NQ];            // asked for first, added last
+    float w_shared = 0.0f, w_passed = 0.0f;
+    if (p.shared) {
+#pragma unroll
+        for (int k = 0; k < NQ; ++k)
+            shared[k] = i + k * step < width ? __ldcg(reinterpret_cast<const float4*>(p.shared + static_cast<size_t>(row) * p.ld_shared + i + k * step)) : zero;
+        w_shared = p.gate ? __ldcg(p.gate + row) : 1.0f;
+    }
+    if (p.identity) {
+        w_passed = __ldcg(p.identity + row);
+#pragma unroll
+        for (int k = 0; k < NQ; ++k) {
+            passed[k] = zero;
+            if (i + k * step >= width) continue;
+            float e[4];
+            const size_t at = static_cast<size_t>(row) * p.ld_x + i + k * step;
+            if (p.x_bf16) mlr_load4(static_cast<const __nv_bfloat16*>(p.x) + at, e);
+            else mlr_load4(static_cast<const float*>(p.x) + at, e);
+            passed[k] = make_float4(e[0], e[1], e[2], e[3]);
+        }
+    }
+#pragma unroll 4
+    for (int j = 0; j < p.top; ++j) {
+        const long long from = s.from[j];
+        float4 e[NQ];
+#pragma unroll
+        for (int k = 0; k < NQ; ++k) e[k] = from >= 0 && i + k * step < width ? __ldcg(reinterpret_cast<const float4*>(p.y + from + i + k * step)) : zero;
+        if (from >= 0) add(s.weight[j], e);
+    }
+    if (p.identity) add(w_passed, passed);
+    if (p.shared) add(w_shared, shared);
+}
+
 static int check_pieces(const Pieces& p, int width, const char* who) {
     MLR_REQUIRE(p.top >= 1 && p.top <= kMaxPieces && p.row_of_pair && p.weights && p.ldy >= width && (!p.shared || p.ld_shared >= width) &&
                     (!p.identity || (p.x && p.ld_x >= width)),

@@ -33,6 +33,7 @@ template <typename TO, int S, int V>
 __global__ void __launch_bounds__(kThreads) streams_step_kernel(float* h, const float* y, long long ld_y, const float* y_scale, const float* mix,
                                                                  const float* w_out, const float* w_in, const float* norm_weight, float eps,
                                                                  TO* out, long long ld_out, const int* rows, int width, int streams_given, Pieces pieces) {
+    mlr_grid_dependents_may_start();
     mlr_grid_wait();
     __shared__ StagedPieces staged;
     extern __shared__ __align__(16) float u[];          // [width]
@@ -134,10 +135,7 @@ __global__ void __launch_bounds__(kThreads) streams_step_kernel(float* h, const 
             }
         }
     }
-    if (!out) {
-        mlr_grid_dependents_may_start();
-        return;
-    }
+    if (!out) return;
     const float inv = 1.0f / sqrtf(mlr_block_sum(squares, scratch) / static_cast<float>(width) + eps);
     TO* orow = out + static_cast<size_t>(blockIdx.x) * ld_out;
     for (int c = threadIdx.x * V; c < width; c += kThreads * V) {         // a thread's own columns
@@ -147,7 +145,95 @@ __global__ void __launch_bounds__(kThreads) streams_step_kernel(float* h, const 
         for (int e = 0; e < V; ++e) value[e] = u[c + e] * inv * (norm_weight ? weight[e] : 1.0f);
         mlr_store_group<V>(orow + c, value);
     }
+}
+
+// The same for 1 to 4 copies of at most NQ * 1024 columns, four at a time: a thread keeps its columns in registers and asks for
+// all of them (every copy, the result or its pieces) before it uses the first.  The kernel above goes back to memory for every group of
+// columns, which the few rows of a decode step pay in full: one row of 4096 with pieces 10.2 -> 5.2 us, three rows of 4 x 2048 6.0 -> 4.4 us, 3863 rows of those 67 -> 60 us.
+template <typename TO, int S, int NQ>
+__global__ void __launch_bounds__(kThreads) streams_step_quads_kernel(float* h, const float* y, long long ld_y, const float* y_scale, const float* mix,
+                                                                       const float* w_out, const float* w_in, const float* norm_weight, float eps,
+                                                                       TO* out, long long ld_out, const int* rows, int width, Pieces pieces) {
     mlr_grid_dependents_may_start();
+    mlr_grid_wait();
+    __shared__ StagedPieces staged;
+    __shared__ float scratch[32];
+    constexpr int kStep = kThreads * 4;
+    const int row = rows ? rows[blockIdx.x] : blockIdx.x;
+    const bool writes = y || pieces.y;
+    const int c0 = threadIdx.x * 4;
+    const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    auto load = [&](const float* p, float4 (&v)[NQ]) {
+#pragma unroll
+        for (int k = 0; k < NQ; ++k) v[k] = c0 + k * kStep < width ? __ldcg(reinterpret_cast<const float4*>(p + c0 + k * kStep)) : zero;
+    };
+    auto add = [](float4& v, float w, const float4& a) {
+        v.x = fmaf(w, a.x, v.x); v.y = fmaf(w, a.y, v.y); v.z = fmaf(w, a.z, v.z); v.w = fmaf(w, a.w, v.w);
+    };
+    float* x = h + static_cast<size_t>(row) * S * width;
+    float4 old[S][NQ], u[NQ];
+#pragma unroll
+    for (int s = 0; s < S; ++s) load(x + static_cast<size_t>(s) * width, old[s]);
+    float in[S];
+#pragma unroll
+    for (int s = 0; s < S; ++s) in[s] = w_in ? w_in[s] : 1.0f;
+#pragma unroll
+    for (int k = 0; k < NQ; ++k) u[k] = zero;
+    if (writes) {
+        float4 result[NQ];
+        if (pieces.y) {
+            stage_pieces(pieces, row, staged);
+            __syncthreads();
+            piece_sums<NQ>(pieces, staged, row, c0, kStep, width, result);
+        } else {
+            load(y + static_cast<size_t>(row) * ld_y, result);
+        }
+        if (y_scale) {
+            float4 scale[NQ];
+            load(y_scale, scale);
+#pragma unroll
+            for (int k = 0; k < NQ; ++k) { result[k].x *= scale[k].x; result[k].y *= scale[k].y; result[k].z *= scale[k].z; result[k].w *= scale[k].w; }
+        }
+#pragma unroll
+        for (int t = 0; t < S; ++t) {
+            const float o = w_out[t];
+            float m[S];
+#pragma unroll
+            for (int s = 0; s < S; ++s) m[s] = mix[s * S + t];
+#pragma unroll
+            for (int k = 0; k < NQ; ++k) {
+                float4 value = zero;
+#pragma unroll
+                for (int s = 0; s < S; ++s) add(value, m[s], old[s][k]);
+                add(value, o, result[k]);
+                add(u[k], in[t], value);
+                if (c0 + k * kStep < width) *reinterpret_cast<float4*>(x + static_cast<size_t>(t) * width + c0 + k * kStep) = value;
+            }
+        }
+    } else {
+#pragma unroll
+        for (int s = 0; s < S; ++s)
+#pragma unroll
+            for (int k = 0; k < NQ; ++k) add(u[k], in[s], old[s][k]);
+    }
+    if (!out) return;
+    float4 weight[NQ];
+    if (norm_weight) load(norm_weight, weight);
+    float squares = 0.0f;
+#pragma unroll
+    for (int k = 0; k < NQ; ++k) {
+        squares = fmaf(u[k].x, u[k].x, squares); squares = fmaf(u[k].y, u[k].y, squares);
+        squares = fmaf(u[k].z, u[k].z, squares); squares = fmaf(u[k].w, u[k].w, squares);
+    }
+    const float inv = 1.0f / sqrtf(mlr_block_sum(squares, scratch) / static_cast<float>(width) + eps);
+    TO* orow = out + static_cast<size_t>(blockIdx.x) * ld_out;
+#pragma unroll
+    for (int k = 0; k < NQ; ++k) {
+        if (c0 + k * kStep >= width) continue;
+        float value[4] = {u[k].x * inv, u[k].y * inv, u[k].z * inv, u[k].w * inv};
+        if (norm_weight) { value[0] *= weight[k].x; value[1] *= weight[k].y; value[2] *= weight[k].z; value[3] *= weight[k].w; }
+        mlr_store_group<4>(orow + c0 + k * kStep, value);
+    }
 }
 
 template <typename T>
@@ -215,6 +301,31 @@ int streams_step(float* h, const float* y, long long ld_y, const float* y_scale,
     const auto aligned = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
     const bool wide = width % 4 == 0 && aligned(h) && aligned(y) && ld_y % 4 == 0 && aligned(y_scale) && aligned(norm_weight) && aligned(out) &&
                       ld_out % 4 == 0 && (!pieces.y || pieces_aligned(pieces));
+    // A thread's columns in registers: up to 4 copies of up to 4096 columns (64 registers of stream).
+    const bool quads = wide && streams <= 4 && width <= 4 * 4 * kThreads;
+#define MLR_QUADS(TO, S, NQ)                                                                                                               \
+    mlr_launch((streams_step_quads_kernel<TO, S, NQ>), dim3(count), dim3(kThreads), 0, stream, h, y, ld_y, y_scale, mix, w_out, w_in,        \
+               norm_weight, eps, static_cast<TO*>(out), ld_out, rows, width, pieces)
+#define MLR_PER(TO, S)                                           \
+    do {                                                         \
+        if (width <= 4 * kThreads) MLR_QUADS(TO, S, 1);          \
+        else if (width <= 8 * kThreads) MLR_QUADS(TO, S, 2);     \
+        else MLR_QUADS(TO, S, 4);                                \
+    } while (0)
+#define MLR_COPIES(TO)                   \
+    switch (streams) {                   \
+        case 1: MLR_PER(TO, 1); break;   \
+        case 2: MLR_PER(TO, 2); break;   \
+        case 3: MLR_PER(TO, 3); break;   \
+        default: MLR_PER(TO, 4); break;  \
+    }
+    if (quads) {
+        if (out_bf16) { MLR_COPIES(__nv_bfloat16) } else { MLR_COPIES(float) }
+        return mlr_launched("streams_step");
+    }
+#undef MLR_COPIES
+#undef MLR_PER
+#undef MLR_QUADS
 #define MLR_GO(TO, S, V)                                                                                                                   \
     do {                                                                                                                                   \
         if (shared > 48 * 1024)                                                                                                            \

@@ -34,7 +34,8 @@
 //    memory: a lane needs 16 bytes of its token's row per 512 values of K, eight registers' worth of loads, and
 //    shared memory is all ring (three slots at any row count).  A product that ADDS into the stream is cut along K
 //    into parts of at most 4096 values for that: each part adds its partial product into the stream (a cell has the
-//    same owner in every part).  Other products (a norm prologue, a wider K) stage their activations in shared
+//    same owner in every part).  So is one that stores float32: its first part stores, the others add (4096 x 12288
+//    at one row: 20 us, against 65 us for 32 blocks of the one-block tcgen05 kernel).  Other products (a norm prologue, a wider K) stage their activations in shared
 //    memory beside a ring of two slots (three at one row), with shorter copies or one buffer of partial sums
 //    where room is short.
 //  * Every block needs all of a product's activations, so 148 blocks reading eight float32 rows of the
@@ -51,6 +52,7 @@
 // The reference sends these products to cuBLAS gemv kernels (src/minillm/cuda/matrix.cpp:30-36) and
 // runs norm, gate and residual add as kernels of their own (src/minillm/cuda/layer.cpp:42-70).
 #include "common.cuh"
+#include "weight_ring.cuh"
 
 namespace {
 
@@ -66,7 +68,6 @@ constexpr int kGateBlock = 128;
 constexpr int kMaxParts = 16;
 constexpr int kMaxRows = 8;
 constexpr int kPartialBytes = kConsumerWarps * kUnitRows * kMaxRows * 4;        // one buffer of the warps' partial sums
-constexpr long long kWaitLimitCycles = 4000000000LL;      // about two seconds
 
 enum Mode : int { kStoreBf16 = 0, kStoreF32 = 1, kAddF32 = 2, kSiluGateBf16 = 3, kSquaredReluBf16 = 4 };
 
@@ -104,55 +105,6 @@ struct Job {
     int* status;
 };
 
-__device__ __forceinline__ void mma_16x8x16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};\n"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ uint4 load_shared16(uint32_t address) {
-    uint4 v;
-    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];\n" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(address));
-    return v;
-}
-
-// ---- mbarriers and bulk copies (the ring of weights)
-__device__ __forceinline__ void mbar_init(uint32_t bar, int count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(bar), "r"(count));
-}
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
-    uint32_t done;
-    asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
-                 : "=r"(done)
-                 : "r"(bar), "r"(parity)
-                 : "memory");
-    return done != 0;
-}
-__device__ __forceinline__ void bulk_copy(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(dst), "l"(src),
-                 "r"(bytes), "r"(bar)
-                 : "memory");
-}
-// Waits for a phase of a barrier, but not for ever.  A wait that runs out (about two seconds) sets the block's
-// `failed` flag and MLR_STATUS_TIMEOUT; from then on no wait of the block waits, so that every thread still walks
-// through the same barriers to the kernel's end (its results are then worthless, and the status says so).
-__device__ __forceinline__ void wait_phase(uint32_t bar, uint32_t parity, volatile int* failed, int* status) {
-    if (mbar_try_wait(bar, parity)) return;
-    const long long start = clock64();
-    while (!mbar_try_wait(bar, parity)) {
-        if (*failed) return;
-        if (clock64() - start > kWaitLimitCycles) {
-            *failed = 1;
-            if (status) atomicOr(status, MLR_STATUS_TIMEOUT);
-            return;
-        }
-    }
-}
 __device__ __forceinline__ void consumers_sync() { asm volatile("bar.sync 2, %0;\n" ::"n"(kConsumers) : "memory"); }
 
 // Row `r` (0..15) of unit `unit` in W: rows 16 u .. 16 u + 15 of a plain matrix; in a stacked gate/up matrix the gate
@@ -167,10 +119,6 @@ __device__ __forceinline__ int row_of_unit(const Link& l, int unit, int r) {
 __host__ __device__ inline int units_of(const Link& l) {
     return l.mode == kSiluGateBf16 ? l.N / kUnitRows : (l.N + kUnitRows - 1) / kUnitRows;
 }
-// Bytes between rows of the activations in shared memory, and between a slot's rows of weights: the values and a
-// pad that makes it 64 modulo 128, so that the 16-byte reads of the eight rows a quarter-warp touches fall into
-// different banks.
-__host__ __device__ inline int pitch_bytes(int values) { return values * 2 + ((64 - (values * 2) % 128) + 128) % 128; }
 __host__ __device__ inline size_t x_region_bytes(int M, int K) { return (static_cast<size_t>(M) * pitch_bytes(K) + 127) / 128 * 128; }
 __host__ __device__ inline size_t ring_bytes(int chunk, int slots) { return static_cast<size_t>(slots) * kUnitRows * pitch_bytes(chunk); }
 
@@ -489,10 +437,10 @@ int slots_for(size_t x_bytes, int chunk) {
 }
 
 // How many parts a product over K values is cut into for M rows (1: it stays whole), and the width of a part.  Only a
-// product that adds into the stream can be cut; it is, when its activations would push the ring below its best size.
+// product that adds into the stream or stores float32 can be cut; it is, when its activations would push the ring below its best size.
 // Whether a product keeps its activations in registers: its norm, if any, was prepared, and its K (or, for a product
-// that adds into the stream, the K of its parts) is at most 512 * kRegisterBlocks.
-bool in_registers(int K, int mode, int norm) { return norm != 1 && (mode == kAddF32 || K <= 512 * kRegisterBlocks); }
+// that adds into the stream or stores float32, the K of its parts) is at most 512 * kRegisterBlocks.
+bool in_registers(int K, int mode, int norm) { return norm != 1 && (mode == kAddF32 || (mode == kStoreF32 && norm == 0) || K <= 512 * kRegisterBlocks); }
 
 int parts_of(int M, int K, int mode, int norm, int& part_width) {
     part_width = K;
@@ -544,6 +492,7 @@ int launch(const Link& l, int M, int* status, cudaStream_t stream) {
             p.W = l.W + from;
             p.x = static_cast<const __nv_bfloat16*>(l.x) + from;
             p.K = l.K - from < width ? l.K - from : width;
+            if (part > 0 && p.mode == kStoreF32) p.mode = kAddF32;                       // the first part stores, the others add to it
             if (part + 1 < job.n_parts) p.side = nullptr, p.squares = nullptr;       // the last part has the stream's final values
         }
     }
@@ -587,8 +536,8 @@ int launch(const Link& l, int M, int* status, cudaStream_t stream) {
 
 }  // namespace
 
-// Whether mlr_gemv_bf16 takes a product of `M` rows over K values that does not add into the stream (its activations
-// must fit shared memory beside the ring; a product that adds is cut into parts that do).
+// Whether mlr_gemv_bf16 takes a product of `M` rows over K values that neither adds into the stream nor stores float32 (its
+// activations must fit shared memory beside the ring; those two are cut into parts that do).
 MLR_API int mlr_gemv_bf16_fits(int M, int K) {
     return M >= 1 && M <= kMaxRows && K >= 8 && K % 8 == 0 && (K <= 512 * kRegisterBlocks || chunk_for(x_region_bytes(M, K), 1) > 0);
 }

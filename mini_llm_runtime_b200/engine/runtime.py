@@ -268,8 +268,8 @@ class Runtime:
 
     # ---- few rows: a pass over the weights with the neighbouring row-wise work folded in
     def _gemv_fits(self, K: int, adds: bool = False) -> bool:
-        """Whether the few-row kernel takes `gemv_rows` rows of K values (a product that adds into the stream is cut
-        along K until it does)."""
+        """Whether the few-row kernel takes `gemv_rows` rows of K values (a product that adds into the stream or stores
+        float32, `adds`, is cut along K until it does)."""
         key = (min(self.gemv_rows, 8), K, adds)
         if key not in self._gemv_fit:
             self._gemv_fit[key] = K % 8 == 0 and (adds or bool(native.module("gemv_bf16").mlr_gemv_bf16_fits(key[0], K)))
@@ -281,7 +281,7 @@ class Runtime:
         return self.dtype is torch.bfloat16 and self.gemv_rows > 0 and self._gemv_fits(width) and b.le(count, min(self.gemv_rows, 8))
 
     def _gemv(self, b, x: Buf, w: torch.Tensor, adds: bool = False) -> bool:
-        """Whether this bf16 product (`adds`: into the float32 stream) is a few-row pass over the weights."""
+        """Whether this bf16 product (`adds`: one that adds into the stream or stores float32) is a few-row pass over the weights."""
         if (self.dtype is not torch.bfloat16 or self.gemv_rows <= 0 or w.dtype is not torch.bfloat16
                 or not self._gemv_fits(w.shape[1], adds and x.norm is None)):
             return False
@@ -344,7 +344,7 @@ class Runtime:
         N, K = w.shape
         if out is None:
             out = b.temp(x.rows, N, torch.float32 if self.dtype is torch.float32 else out_dtype)
-        if self._gemv(b, x, w):
+        if self._gemv(b, x, w, adds=out.dtype is torch.float32 and w.shape[1] <= 16 * 4096):
             self._gemv_launch(b, x, w, out, "bf16" if out.dtype is torch.bfloat16 else "f32")
             return out
         x = self.materialize(b, x)

@@ -252,6 +252,16 @@ def test_gemv_bf16_and_what_it_folds_in(M, N, K):
             assert torch.allclose(got.cpu().double(), want_n, atol=3e-2, rtol=3e-2), (got.cpu().double() - want_n).abs().max()
 
 
+@pytest.mark.parametrize("M,N,K", [(1, 4096, 12288), (8, 40, 4104), (8, 301, 12288), (3, 17, 16384)])
+def test_gemv_bf16_stores_float32_of_a_wide_k_in_parts(M, N, K):
+    x = torch.randn(M, K, generator=gen(1)).to(torch.bfloat16)
+    w = (torch.randn(N, K, generator=gen(2)) * K ** -0.5).to(torch.bfloat16)
+    out = torch.full((M, N), float("nan"), device=DEV)
+    F().gemv_bf16(w.to(DEV), x.to(DEV), out, "f32")
+    # float32 sums of K products whose total is of size 1
+    assert torch.allclose(out.cpu().double(), x.double() @ w.double().T, atol=1e-4, rtol=1e-4)
+
+
 @pytest.mark.parametrize("M,inter,K", [(1, 256, 128), (4, 12288, 4096), (3, 300, 104), (8, 1000, 512), (8, 640, 5120)])
 def test_gemv_bf16_gate(M, inter, K):
     """silu(gate) * up in the epilogue, over the stacked operand the feed-forward keeps (blocks of 128 gate

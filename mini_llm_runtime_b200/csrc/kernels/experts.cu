@@ -23,6 +23,7 @@
 // (`gated` 2): g <- min(g, limit), u <- clamp(u, -limit, limit) where limit > 0, then g * sigmoid(alpha g) * (u + up_offset).
 #include "common.cuh"
 #include "pieces.cuh"
+#include "weight_ring.cuh"
 
 #include <climits>
 
@@ -75,6 +76,13 @@ __global__ void __launch_bounds__(kRouteThreads) route_kernel(const T* x, long l
                                                               int rows, int width, int experts, int routed, int groups, int keep, int top,
                                                               int has_gate, int* chosen, float* weights, int* place, int* counts, float* shared_gate,
                                                               float* identity, int kind) {
+    mlr_grid_dependents_may_start();
+    if (ROWS == 1) {
+        // A step of few rows: its router has left the cache since the step before.  It is on its way before the wait.
+        const char* matrix = reinterpret_cast<const char*>(router);
+        const size_t bytes = static_cast<size_t>(experts + has_gate) * width * sizeof(float);
+        for (size_t at = threadIdx.x * 128; at < bytes; at += blockDim.x * 128) asm volatile("prefetch.global.L2 [%0];\n" ::"l"(matrix + at));
+    }
     mlr_grid_wait();
     extern __shared__ __align__(16) float shared[];
     float* xs = shared;                                 // [ROWS][width]
@@ -95,7 +103,7 @@ __global__ void __launch_bounds__(kRouteThreads) route_kernel(const T* x, long l
         if (width % 4 == 0) {         // 16 bytes at a time (rows of the router and the shared rows start on 16-byte borders then)
             const float4* w4 = reinterpret_cast<const float4*>(w);
             const float4* x4 = reinterpret_cast<const float4*>(xs);
-#pragma unroll 4
+#pragma unroll ROWS == 1 ? 8 : 4
             for (int c = lane; c < width / 4; c += 32) {
                 const float4 a = w4[c];
 #pragma unroll
@@ -209,6 +217,7 @@ __global__ void __launch_bounds__(kRouteThreads) route_kernel(const T* x, long l
 // (the row of pair = token * top + choice in the order by expert), pair_of_row [pairs] the other way.
 __global__ void __launch_bounds__(1024) arrange_kernel(int* counts, const int* chosen, const int* place, int experts, int pairs, int tile_rows,
                                                        int* first_row, int* tiles, int* n_tiles, int* row_of_pair, int* pair_of_row) {
+    mlr_grid_dependents_may_start();
     mlr_grid_wait();
     __shared__ int first[kMaxExperts + 1];
     __shared__ int first_tile[kMaxExperts + 1];
@@ -466,6 +475,146 @@ __global__ void __launch_bounds__(256) expert_product_mma_kernel(const __nv_bflo
         }
 }
 
+// ---- the same product for steps of up to eight rows: a pass over the chosen experts' weights ----
+// An expert then has at most eight rows, and the product is bound by the reading of its weights.  One warp of a block keeps a ring of
+// slots filled with the weights of 16 rows (a unit; with DUAL 8 rows of each matrix, whose outputs are gated together) by bulk
+// copies of up to 4 KB, 16 warps multiply: warp w takes values 32 w .. 32 w + 31 of every 512 of K, the expert's rows are the second
+// operand of `mma.sync.m16n8k16` and stay in registers while the block's units are of one expert (a block's units are neighbours).
+// The warps' sums are added in warp order, so a result does not depend on the grid or on what else the step holds.  The tiled
+// kernel above left most of the memory's rate unused at these sizes (a third of the SMs had no block, a block 28 KB on their way):
+// gate/up and down of one row with 4 of 20 outputs at 2048 x 4096: 77 -> 20 and 38 -> 12 us; of three rows with 4 of 16 at 1024 x 2048: 41 -> 16
+// and 19 -> 12 us.
+constexpr int kFewRows = 8, kFewWarps = 16, kFewConsumers = kFewWarps * 32, kFewThreads = kFewConsumers + 32;
+constexpr int kFewUnit = 16;                  // rows of weights a unit has
+constexpr int kFewChunk = 2048;               // values of K of a unit in one slot, at most
+constexpr int kFewBlocks = 8;                 // blocks of 512 values of K a lane keeps of its row of activations: K <= 4096
+constexpr int kFewMostSlots = 8;
+constexpr int kFewMostTiles = kFewRows * kMaxTop;
+constexpr int kFewPartial = kFewWarps * kFewUnit * kFewRows;          // floats of one buffer of the warps' sums
+
+template <typename TO, bool DUAL>
+__global__ void __launch_bounds__(kFewThreads, 1) expert_few_kernel(const __nv_bfloat16* a, long long lda, const int* source, int divisor,
+                                                                    const __nv_bfloat16* w, const __nv_bfloat16* w2, int N, int K, TO* out,
+                                                                    long long ldo, const int* tiles, const int* n_tiles, ExpertGate shape, int chunk,
+                                                                    int slots, int* status) {
+    extern __shared__ __align__(128) unsigned char ring_and_sums[];
+    __shared__ __align__(8) unsigned long long barriers[2 * kFewMostSlots];
+    __shared__ int tile_of[3 * kFewMostTiles];
+    __shared__ int failed_flag;
+    float* partial = reinterpret_cast<float*>(ring_and_sums);              // [2][16 warps][16 rows][8 tokens]
+    const int pitch = pitch_bytes(chunk), slot_bytes = kFewUnit * pitch;
+    const uint32_t ring = static_cast<uint32_t>(__cvta_generic_to_shared(ring_and_sums)) + 2 * kFewPartial * 4;
+    const uint32_t bars = static_cast<uint32_t>(__cvta_generic_to_shared(barriers));
+    auto full_bar = [&](int slot) { return bars + 8u * slot; };
+    auto empty_bar = [&](int slot) { return bars + 8u * (kFewMostSlots + slot); };
+    volatile int* failed = &failed_flag;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    mlr_grid_dependents_may_start();
+    if (threadIdx.x == 0) {
+        failed_flag = 0;
+        for (int s = 0; s < slots; ++s) {
+            mbar_init(full_bar(s), 1);
+            mbar_init(empty_bar(s), kFewWarps);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+    }
+    mlr_grid_wait();
+    const int n = min(__ldcg(n_tiles), kFewMostTiles);
+    for (int i = threadIdx.x; i < 3 * n; i += kFewThreads) tile_of[i] = __ldcg(tiles + i);
+    __syncthreads();
+    constexpr int kOutputs = DUAL ? kFewUnit / 2 : kFewUnit;              // of a unit
+    const int per_tile = (N + kOutputs - 1) / kOutputs, units = n * per_tile;
+    const int first = static_cast<int>(static_cast<long long>(units) * blockIdx.x / gridDim.x);
+    const int last = static_cast<int>(static_cast<long long>(units) * (blockIdx.x + 1) / gridDim.x);
+    const int chunks = (K + chunk - 1) / chunk;
+
+    if (warp == kFewWarps) {
+        int i = 0;
+        for (int unit = first; unit < last; ++unit) {
+            const int expert = tile_of[3 * (unit / per_tile)], r = lane & 15;
+            const int row = unit % per_tile * kOutputs + r % kOutputs;
+            const bool valid = lane < kFewUnit && row < N;
+            const int n_valid = __popc(__ballot_sync(0xffffffffu, valid));
+            const __nv_bfloat16* src = (DUAL && r >= kOutputs ? w2 : w) + (static_cast<size_t>(expert) * N + (valid ? row : 0)) * K;
+            for (int c = 0; c < chunks; ++c, ++i) {
+                const int slot = i % slots;
+                if (i >= slots) wait_phase(empty_bar(slot), ((i / slots) - 1) & 1, failed, status);
+                const uint32_t bytes = static_cast<uint32_t>(min(chunk, K - c * chunk)) * 2u;
+                if (lane == 0) mbar_expect_tx(full_bar(slot), bytes * n_valid);
+                __syncwarp();
+                if (valid && !*failed) bulk_copy(ring + slot * slot_bytes + lane * pitch, src + c * chunk, bytes, full_bar(slot));
+            }
+        }
+        if (*failed) {
+            // Leave only when the copies that were issued have landed, or after another bounded wait.
+            for (int back = 1; back <= slots && back <= i; ++back) {
+                const int j = i - back;
+                const long long start = clock64();
+                while (!mbar_try_wait(full_bar(j % slots), (j / slots) & 1) && clock64() - start < kWaitLimitCycles) {
+                }
+            }
+        }
+        return;
+    }
+
+    const int g = lane >> 2, t = lane & 3;
+    const uint32_t in_slot = (warp * 32 + t * 8) * 2;
+    const uint4 zero = make_uint4(0, 0, 0, 0);
+    uint4 x[kFewBlocks];
+    int tile = -1, row0 = 0, rows = 0, parity = 0, i = 0;
+    for (int unit = first; unit < last; ++unit) {
+        if (unit / per_tile != tile) {
+            tile = unit / per_tile, row0 = tile_of[3 * tile + 1], rows = min(tile_of[3 * tile + 2], kFewRows);
+            const int r = row0 + min(g, rows - 1);
+            const __nv_bfloat16* row = a + static_cast<long long>(source ? __ldcg(source + r) / divisor : r) * lda;
+#pragma unroll
+            for (int b = 0; b < kFewBlocks; ++b) {
+                const int k = b * 512 + warp * 32 + t * 8;
+                x[b] = g < rows && k < K ? __ldcg(reinterpret_cast<const uint4*>(row + k)) : zero;
+            }
+        }
+        float c[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+        for (int piece = 0; piece < kFewBlocks / 4; ++piece) {          // a slot holds up to four blocks: every register's index is a constant
+            if (piece < chunks) {
+                const int slot = i % slots;
+                wait_phase(full_bar(slot), (i / slots) & 1, failed, status);
+#pragma unroll
+                for (int sub = 0; sub < 4; ++sub) {
+                    const bool in = piece * kFewChunk + sub * 512 + warp * 32 + t * 8 < K;
+                    const uint32_t at = ring + slot * slot_bytes + sub * 1024 + in_slot;
+                    const uint4 upper = in ? load_shared16(at + g * pitch) : zero;
+                    const uint4 lower = in ? load_shared16(at + (g + 8) * pitch) : zero;
+                    const uint4 v = x[piece * 4 + sub];
+                    mma_16x8x16(c, upper.x, lower.x, upper.y, lower.y, v.x, v.y);
+                    mma_16x8x16(c, upper.z, lower.z, upper.w, lower.w, v.z, v.w);
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(empty_bar(slot));
+                ++i;
+            }
+        }
+        // The warps' sums meet in shared memory; 128 threads add them in warp order (two buffers: the next unit does not wait for this).
+        float* sums = partial + parity * kFewPartial;
+        float* mine = sums + warp * kFewUnit * kFewRows;
+        *reinterpret_cast<float2*>(mine + g * kFewRows + 2 * t) = make_float2(c[0], c[1]);
+        *reinterpret_cast<float2*>(mine + (g + 8) * kFewRows + 2 * t) = make_float2(c[2], c[3]);
+        asm volatile("bar.sync 1, %0;\n" ::"n"(kFewConsumers) : "memory");
+        if (threadIdx.x < kOutputs * kFewRows) {
+            const int r = threadIdx.x % kOutputs, m = threadIdx.x / kOutputs, col = unit % per_tile * kOutputs + r;
+            float y = 0.0f, up = 0.0f;
+#pragma unroll
+            for (int v = 0; v < kFewWarps; ++v) {
+                y += sums[(v * kFewUnit + r) * kFewRows + m];
+                if (DUAL) up += sums[(v * kFewUnit + r + kOutputs) * kFewRows + m];
+            }
+            if (m < rows && col < N) mlr_store(out + static_cast<size_t>(row0 + m) * ldo, col, DUAL ? expert_gate(y, up, shape) : y);
+        }
+        parity ^= 1;
+    }
+}
+
 template <bool VEC>
 __global__ void __launch_bounds__(256) combine_kernel(Pieces pieces, float* out, long long ldo, int width) {
     mlr_grid_wait();
@@ -608,6 +757,45 @@ MLR_API int mlr_experts_product(const void* a, long long lda, int act_bf16, cons
     }
 #undef MLR_GO
     return mlr_launched("experts_product");
+}
+
+// Whether `mlr_experts_product_few` takes products over K values from rows `lda` apart: 1 yes, 0 no.
+MLR_API int mlr_experts_few(int K, long long lda) { return K >= 8 && K <= 512 * kFewBlocks && mlr_experts_tensor_cores(K, lda); }
+
+// The same for steps of at most 8 rows in bfloat16 (a tile of `tiles` is then all rows of one expert): out is bfloat16 with a gate and float32
+// without.  `status`: a device word in which a wait that ran out sets MLR_STATUS_TIMEOUT.
+MLR_API int mlr_experts_product_few(const void* a, long long lda, const int* source, int divisor, const void* w, const void* w2, int gated, int N,
+                                    int K, void* out, long long ldo, const int* tiles, const int* n_tiles, int rows, int top, float alpha, float limit,
+                                    float up_offset, int* status, cudaStream_t stream) {
+    MLR_REQUIRE(gated >= 0 && gated <= 2, "experts_product: unknown gate %d", gated);
+    MLR_REQUIRE(a && w && out && tiles && n_tiles && N > 0 && (!gated || w2) && (!source || divisor > 0), "experts_product: bad arguments");
+    const auto aligned = [](const void* q) { return reinterpret_cast<uintptr_t>(q) % 16 == 0; };
+    MLR_REQUIRE(rows <= kFewRows && top >= 1 && top <= kMaxTop && K >= 8 && K <= 512 * kFewBlocks && K % 8 == 0 && lda % 8 == 0 && aligned(a) &&
+                    aligned(w) && (!gated || aligned(w2)),
+                "experts_product: up to %d rows of up to %d values on 16-byte borders", kFewRows, 512 * kFewBlocks);
+    if (rows <= 0) return 0;
+    const ExpertGate shape = {gated, alpha, limit, up_offset};
+    const int chunk = K >= kFewChunk ? kFewChunk : (K + 511) / 512 * 512;
+    const int slot_bytes = kFewUnit * pitch_bytes(chunk), sums = 2 * kFewPartial * 4;
+    int room = 0, device = 0;
+    cudaGetDevice(&device);
+    cudaDeviceGetAttribute(&room, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+    room -= 8192 + sums;                        // the kernel's static shared memory and what the driver keeps
+    int slots = room / slot_bytes;
+    if (slots > kFewMostSlots) slots = kFewMostSlots;
+    MLR_REQUIRE(slots >= 2, "experts_product: no room for the ring of weights");
+    const int bytes = sums + slots * slot_bytes;
+    const __nv_bfloat16 *ab = static_cast<const __nv_bfloat16*>(a), *wb = static_cast<const __nv_bfloat16*>(w), *w2b = static_cast<const __nv_bfloat16*>(w2);
+    if (gated) {
+        cudaFuncSetAttribute(expert_few_kernel<__nv_bfloat16, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        mlr_launch((expert_few_kernel<__nv_bfloat16, true>), dim3(mlr_sm_count()), dim3(kFewThreads), bytes, stream, ab, lda, source, divisor, wb, w2b,
+                   N, K, static_cast<__nv_bfloat16*>(out), ldo, tiles, n_tiles, shape, chunk, slots, status);
+    } else {
+        cudaFuncSetAttribute(expert_few_kernel<float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        mlr_launch((expert_few_kernel<float, false>), dim3(mlr_sm_count()), dim3(kFewThreads), bytes, stream, ab, lda, source, divisor, wb, w2b, N, K,
+                   static_cast<float*>(out), ldo, tiles, n_tiles, shape, chunk, slots, status);
+    }
+    return mlr_launched("experts_product_few");
 }
 
 // The same tensor-core product for `count` matrices that all take the same rows (the heads of a per-head projection):

@@ -127,12 +127,21 @@ class RoutedExperts(FeedForward):
         b.launch("experts", "mlr_experts_arrange", self.counts.data_ptr(), chosen.ptr, place.ptr, E, rows, top, tile_rows, first_row.ptr,
                  tiles.ptr, n_tiles.ptr, row_of_pair.ptr, pair_of_row.ptr, b.stream)
         act = b.temp(rows, top * self.inter, rt.dtype)             # [rows * top, inter], rows in the order by expert
-        b.launch("experts", "mlr_experts_product", x.ptr, x.ld, x.is_bf16, pair_of_row.ptr, top, self.w_gate.data_ptr(),
-                 self.w_up.data_ptr(), self.gate_kind, self.inter, self.width, act.ptr, self.inter, int(not rt.is_bf16), tiles.ptr, n_tiles.ptr,
-                 rows, top, E, tile_rows, self.alpha, self.limit, self.up_offset, b.stream)
         y = b.temp(rows, top * self.width, f32)
-        b.launch("experts", "mlr_experts_product", act.ptr, self.inter, x.is_bf16, None, 1, self.w_down.data_ptr(), None, 0, self.width,
-                 self.inter, y.ptr, self.width, 1, tiles.ptr, n_tiles.ptr, rows, top, E, tile_rows, 0.0, 0.0, 0.0, b.stream)
+        # A decode step's few rows are a pass over the chosen experts' weights.
+        few = bool(both) and b.le(rows, 8)
+
+        def product(a, lda, source, divisor, w, w2, kind, N, K, out, out_f32, shape):
+            if few and lib.mlr_experts_few(K, lda):
+                b.launch("experts", "mlr_experts_product_few", a, lda, source, divisor, w, w2, kind, N, K, out, N, tiles.ptr, n_tiles.ptr, rows, top,
+                         *shape, b.status, b.stream)
+            else:
+                b.launch("experts", "mlr_experts_product", a, lda, x.is_bf16, source, divisor, w, w2, kind, N, K, out, N, out_f32, tiles.ptr,
+                         n_tiles.ptr, rows, top, E, tile_rows, *shape, b.stream)
+
+        product(x.ptr, x.ld, pair_of_row.ptr, top, self.w_gate.data_ptr(), self.w_up.data_ptr(), self.gate_kind, self.inter, self.width, act.ptr,
+                int(not rt.is_bf16), (self.alpha, self.limit, self.up_offset))
+        product(act.ptr, self.inter, None, 1, self.w_down.data_ptr(), None, 0, self.width, self.inter, y.ptr, 1, (0.0, 0.0, 0.0))
         shared = None
         if self.shared_inter and self.gate_kind == 2:
             both = rt.linear(b, x, self.shared_gate_up, activation=True)

@@ -1,0 +1,64 @@
+"""Products of routed experts: the pass over the weights of a step's few rows.  Against 64 bits.
+
+Tolerances: operands are bfloat16 and taken as they are, sums are float32: 1e-4 of the results' size (about 1) covers 4096 terms; a
+bfloat16 result is rounded by at most 2^-9 of its value."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _call(module, name, *args):
+    from mini_llm_runtime_b200.ops import native
+    native.call(module, name, *args)
+
+
+def _listed(choices, experts, tile_rows):
+    """choices [rows, top] (an expert past the last: none).  Tiles, their number, the pairs in the order by expert."""
+    tiles, order = [], []
+    for e in range(experts):
+        pairs = (choices.flatten() == e).nonzero().flatten().tolist()
+        for r in range(0, len(pairs), tile_rows):
+            tiles.append((e, len(order) + r, min(tile_rows, len(pairs) - r)))
+        order += pairs
+    on = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    return on(tiles), on([len(tiles)]), order
+
+
+def _gate(g, u, kind, alpha, limit, offset):
+    if kind == 2:
+        g, u = (g.clamp(max=limit), u.clamp(-limit, limit)) if limit > 0 else (g, u)
+        return g * torch.sigmoid(alpha * g) * (u + offset)
+    return g * torch.sigmoid(g) * u
+
+
+@pytest.mark.parametrize("rows,experts,top,N,K,kind", [(1, 1, 1, 8, 8, 1), (1, 16, 4, 1024, 2048, 1), (3, 5, 3, 36, 520, 2), (8, 16, 8, 512, 4096, 2),
+                                                       (8, 2, 1, 300, 1032, 1), (2, 300, 32, 24, 2056, 1)])
+def test_few_rows(rows, experts, top, N, K, kind):
+    from mini_llm_runtime_b200.ops import native
+    g = torch.Generator().manual_seed(rows + N + K)
+    draw = lambda *shape, scale=1.0: (torch.randn(*shape, generator=g) * scale).bfloat16().cuda()
+    x, w, w2 = draw(rows, K + 8)[:, :K], draw(experts, N, K, scale=K ** -0.5), draw(experts, N, K, scale=K ** -0.5)
+    choices = torch.stack([torch.randperm(experts + (top < experts), generator=g)[:top] for _ in range(rows)])
+    choices[0, 0] = 0
+    choices[0, 1:][choices[0, 1:] == 0] = experts
+    tiles, n_tiles, order = _listed(choices, experts, 32)
+    source = torch.tensor(order, dtype=torch.int32, device="cuda")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    shape = (1.702, 0.7, 1.0) if kind == 2 else (0.0, 0.0, 0.0)
+    assert native.module("experts").mlr_experts_few(K, x.stride(0)) == 1
+    act = torch.full((rows * top, N), float("nan"), dtype=torch.bfloat16, device="cuda")
+    _call("experts", "mlr_experts_product_few", x.data_ptr(), x.stride(0), source.data_ptr(), top, w.data_ptr(), w2.data_ptr(), kind, N, K, act.data_ptr(),
+          N, tiles.data_ptr(), n_tiles.data_ptr(), rows, top, *shape, status.data_ptr(), native.stream())
+    gathered = x[source.long() // top]
+    plain = torch.full((rows * top, N), float("nan"), device="cuda")
+    rows_in_order = torch.zeros(rows * top, K, dtype=torch.bfloat16, device="cuda")
+    rows_in_order[:len(order)] = gathered
+    _call("experts", "mlr_experts_product_few", rows_in_order.data_ptr(), K, None, 1, w.data_ptr(), None, 0, N, K, plain.data_ptr(), N, tiles.data_ptr(),
+          n_tiles.data_ptr(), rows, top, 0.0, 0.0, 0.0, status.data_ptr(), native.stream())
+    for e, first, count in tiles.tolist():
+        a = gathered[first:first + count].double()
+        y, up = a @ w[e].double().T, a @ w2[e].double().T
+        assert torch.allclose(plain[first:first + count].double(), y, atol=1e-4, rtol=1e-4)
+        assert torch.allclose(act[first:first + count].double(), _gate(y, up, kind, *shape), atol=1e-3, rtol=4e-3)
+    assert torch.isnan(plain[len(order):]).all() and torch.isnan(act[len(order):].float()).all() and status.item() == 0

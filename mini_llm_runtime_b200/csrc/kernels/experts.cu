@@ -22,6 +22,7 @@
 // weight to `identity` [token] and takes no row of the products.  A second shape of the gate
 // (`gated` 2): g <- min(g, limit), u <- clamp(u, -limit, limit) where limit > 0, then g * sigmoid(alpha g) * (u + up_offset).
 #include "common.cuh"
+#include "expert_gate.cuh"
 #include "pieces.cuh"
 #include "weight_ring.cuh"
 
@@ -35,22 +36,6 @@ constexpr int kMaxTop = 32;
 constexpr int kTileRows = 32;     // rows of one expert per block of a product
 constexpr int kTileCols = 64;
 constexpr int kTileK = 16;
-
-// What the two products of a gated expert become.  kind 1: silu(g) * u.  kind 2: see the head of this file.
-struct ExpertGate {
-    int kind;
-    float alpha, limit, up_offset;
-};
-__device__ __forceinline__ float expert_gate(float g, float u, const ExpertGate& shape) {
-    if (shape.kind == 2) {
-        if (shape.limit > 0.0f) {
-            g = fminf(g, shape.limit);
-            u = fminf(fmaxf(u, -shape.limit), shape.limit);
-        }
-        return g / (1.0f + expf(-shape.alpha * g)) * (u + shape.up_offset);
-    }
-    return g / (1.0f + expf(-g)) * u;
-}
 
 // The index of the largest value that is no NaN, the lowest of equals; 0 where all are NaN.  All lanes of a warp call it and get it.
 __device__ __forceinline__ int warp_argmax(const float* values, int n) {
@@ -615,6 +600,20 @@ __global__ void __launch_bounds__(kFewThreads, 1) expert_few_kernel(const __nv_b
     }
 }
 
+// The rows of the first product side by side in the order by expert, for a kernel that reads them through a tensor map: 16 bytes a thread
+// and step.  It is a pass of its own over pairs * K values (64 MB at 15,452 rows of 2048: 17 us), about a tenth of the products it serves.
+__global__ void __launch_bounds__(256) gather_rows_kernel(const uint4* a, long long ld, const int* source, int divisor, const int* first_row, int experts,
+                                                          uint4* out, int eighths) {
+    mlr_grid_dependents_may_start();
+    mlr_grid_wait();
+    const int rows = __ldcg(first_row + experts);
+    for (int r = blockIdx.x; r < rows; r += gridDim.x) {
+        const uint4* from = a + static_cast<size_t>(__ldcg(source + r) / divisor) * ld;
+        uint4* to = out + static_cast<size_t>(r) * eighths;
+        for (int c = threadIdx.x; c < eighths; c += 256) to[c] = __ldcg(from + c);
+    }
+}
+
 template <bool VEC>
 __global__ void __launch_bounds__(256) combine_kernel(Pieces pieces, float* out, long long ldo, int width) {
     mlr_grid_wait();
@@ -675,10 +674,10 @@ MLR_API int mlr_experts_route(const void* x, long long ld, int act_bf16, const f
 }
 
 // tiles: int32 [3 * (pairs / 32 + experts)]; first_row: int32 [experts + 1]; n_tiles: int32 [1]; row_of_pair, pair_of_row: int32 [pairs].
-// tile_rows: 32, or 64 (the tensor-core products of many rows; the products must be told the same).
+// tile_rows: 32, 64, or 256 for the two-SM product of many rows (`mlr_grouped_product_bf16`); the products must be told the same.
 MLR_API int mlr_experts_arrange(int* counts, const int* chosen, const int* place, int experts, int rows, int top, int tile_rows, int* first_row,
                                 int* tiles, int* n_tiles, int* row_of_pair, int* pair_of_row, cudaStream_t stream) {
-    MLR_REQUIRE(tile_rows == 32 || tile_rows == 64, "experts_arrange: tiles of 32 or 64 rows, not %d", tile_rows);
+    MLR_REQUIRE(tile_rows == 32 || tile_rows == 64 || tile_rows == 256, "experts_arrange: tiles of 32, 64 or 256 rows, not %d", tile_rows);
     MLR_REQUIRE(counts && chosen && place && first_row && tiles && n_tiles && row_of_pair && pair_of_row && experts >= 1 && experts <= kMaxExperts,
                 "experts_arrange: bad arguments");
     if (rows <= 0) return 0;
@@ -757,6 +756,18 @@ MLR_API int mlr_experts_product(const void* a, long long lda, int act_bf16, cons
     }
 #undef MLR_GO
     return mlr_launched("experts_product");
+}
+
+// out [rows * top, K]: row r is row source[r] / top of a (bfloat16, rows `lda` apart), for r < first_row[experts].
+MLR_API int mlr_experts_gather(const void* a, long long lda, const int* source, int rows, int top, const int* first_row, int experts, void* out, int K,
+                               cudaStream_t stream) {
+    MLR_REQUIRE(a && source && top > 0 && first_row && experts >= 1 && out && K > 0 && K % 8 == 0 && lda % 8 == 0 && reinterpret_cast<uintptr_t>(a) % 16 == 0 &&
+                    reinterpret_cast<uintptr_t>(out) % 16 == 0,
+                "experts_gather: rows of multiples of 8 values on 16-byte borders");
+    if (rows <= 0) return 0;
+    mlr_launch(gather_rows_kernel, dim3(mlr_grid_stride_blocks(static_cast<size_t>(rows) * top, 8)), dim3(256), 0, stream, static_cast<const uint4*>(a),
+               lda / 8, source, top, first_row, experts, static_cast<uint4*>(out), K / 8);
+    return mlr_launched("experts_gather");
 }
 
 // Whether `mlr_experts_product_few` takes products over K values from rows `lda` apart: 1 yes, 0 no.

@@ -67,6 +67,8 @@ _SIGNATURES = {
                                   c_int, c_int, c_int, c_int, c_longlong, c_int, c_void_p, c_void_p],
     },
     "gemm_bf16_tcgen05_pair": {
+        "mlr_grouped_product_bf16": [c_void_p, c_longlong, c_int, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_longlong, c_void_p,
+                                     c_void_p, c_float, c_float, c_float, c_void_p, c_void_p],
         "mlr_gemm_bf16_tcgen05_pair": [c_void_p, c_longlong, c_int, c_void_p, c_longlong, c_int, c_int, c_void_p, c_longlong,
                                        c_int, c_void_p, c_void_p],
     },
@@ -154,6 +156,7 @@ _SIGNATURES = {
         "mlr_batched_product_bf16_strided": [c_void_p, c_longlong, c_int, c_void_p, c_void_p, c_longlong, c_int, c_int, c_int, c_int, c_int, c_void_p],
         "mlr_experts_max_tiles": [c_int, c_int],
         "mlr_experts_few": [c_int, c_longlong],
+        "mlr_experts_gather": [c_void_p, c_longlong, c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p],
         "mlr_experts_product_few": [c_void_p, c_longlong, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_longlong, c_void_p,
                                     c_void_p, c_int, c_int, c_float, c_float, c_float, c_void_p, c_void_p],
         "mlr_experts_product": [c_void_p, c_longlong, c_int, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p,

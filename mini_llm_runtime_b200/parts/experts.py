@@ -119,20 +119,27 @@ class RoutedExperts(FeedForward):
         b.launch("experts", "mlr_experts_route", x.ptr, x.ld, x.is_bf16, self.router.data_ptr(), self.correction.data_ptr(), rows,
                  self.width, self.outputs, E, self.groups, self.keep, top, int(self.has_gate), chosen.ptr, weights.ptr, place.ptr,
                  self.counts.data_ptr(), gate.ptr if gate else None, passed.ptr if passed else None, self.router_kind, b.stream)
-        # Tiles of 64 rows for the tensor-core products once an expert gets that many rows on average; 32 otherwise (a decode
+        # Tiles of 256 rows for the two-SM product once an expert gets 64 rows on average; 32 otherwise (a decode
         # step's few rows per expert, the float32 path, rows that do not start on 16-byte borders).
         lib = native.module("experts")
         both = rt.is_bf16 and lib.mlr_experts_tensor_cores(self.width, x.ld) and lib.mlr_experts_tensor_cores(self.inter, self.inter)
-        tile_rows = 64 if both and b.ge(rows, max(1, 64 * E // top)) else 32
+        grouped = bool(both) and rt.use_tcgen05 and b.ge(rows, max(1, 64 * E // top))
+        tile_rows = 256 if grouped else 64 if both and b.ge(rows, max(1, 64 * E // top)) else 32
         b.launch("experts", "mlr_experts_arrange", self.counts.data_ptr(), chosen.ptr, place.ptr, E, rows, top, tile_rows, first_row.ptr,
                  tiles.ptr, n_tiles.ptr, row_of_pair.ptr, pair_of_row.ptr, b.stream)
         act = b.temp(rows, top * self.inter, rt.dtype)             # [rows * top, inter], rows in the order by expert
         y = b.temp(rows, top * self.width, f32)
         # A decode step's few rows are a pass over the chosen experts' weights.
         few = bool(both) and b.le(rows, 8)
+        if grouped:
+            side = b.temp(rows, top * self.width, rt.dtype)        # the rows of the first product side by side
+            b.launch("experts", "mlr_experts_gather", x.ptr, x.ld, pair_of_row.ptr, rows, top, first_row.ptr, E, side.ptr, self.width, b.stream)
 
         def product(a, lda, source, divisor, w, w2, kind, N, K, out, out_f32, shape):
-            if few and lib.mlr_experts_few(K, lda):
+            if grouped:
+                b.launch("gemm_bf16_tcgen05_pair", "mlr_grouped_product_bf16", side.ptr if source is not None else a, K, rows, top, w, w2, E, kind, N, K, out, N,
+                         tiles.ptr, n_tiles.ptr, *shape, b.status, b.stream)
+            elif few and lib.mlr_experts_few(K, lda):
                 b.launch("experts", "mlr_experts_product_few", a, lda, source, divisor, w, w2, kind, N, K, out, N, tiles.ptr, n_tiles.ptr, rows, top,
                          *shape, b.status, b.stream)
             else:

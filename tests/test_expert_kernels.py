@@ -62,3 +62,39 @@ def test_few_rows(rows, experts, top, N, K, kind):
         assert torch.allclose(plain[first:first + count].double(), y, atol=1e-4, rtol=1e-4)
         assert torch.allclose(act[first:first + count].double(), _gate(y, up, kind, *shape), atol=1e-3, rtol=4e-3)
     assert torch.isnan(plain[len(order):]).all() and torch.isnan(act[len(order):].float()).all() and status.item() == 0
+
+
+@pytest.mark.parametrize("rows,experts,top,N,K,kind", [(1, 1, 1, 128, 64, 1), (300, 1, 1, 256, 128, 2), (257, 3, 2, 136, 72, 1), (700, 16, 4, 264, 520, 2),
+                                                       (64, 9, 3, 40, 8, 1)])
+def test_many_rows_on_two_sms(rows, experts, top, N, K, kind):
+    """Tiles that end inside an expert, experts without rows, widths that are no multiple of a tile, rows past the last."""
+    from mini_llm_runtime_b200.ops import native
+    g = torch.Generator().manual_seed(rows + N + K)
+    draw = lambda *shape, scale=1.0: (torch.randn(*shape, generator=g) * scale).bfloat16().cuda()
+    x, w, w2, down = draw(rows, K + 8)[:, :K], draw(experts, N, K, scale=K ** -0.5), draw(experts, N, K, scale=K ** -0.5), draw(experts, K, N, scale=N ** -0.5)
+    choices = torch.stack([torch.randperm(experts + (top < experts), generator=g)[:top] for _ in range(rows)])
+    if experts > 2:
+        choices[choices == 1] = experts              # an expert nobody chose
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    shape = (1.702, 0.7, 1.0) if kind == 2 else (0.0, 0.0, 0.0)
+    tiles, n_tiles, order = _listed(choices, experts, 256)
+    count = len(order)
+    source = torch.tensor(order + [0] * (rows * top - count), dtype=torch.int32, device="cuda")
+    first_row = torch.tensor([(choices < e).sum().item() for e in range(experts)] + [count], dtype=torch.int32, device="cuda")
+    side = torch.full((rows * top, K), float("nan"), dtype=torch.bfloat16, device="cuda")
+    _call("experts", "mlr_experts_gather", x.data_ptr(), x.stride(0), source.data_ptr(), rows, top, first_row.data_ptr(), experts, side.data_ptr(), K,
+          native.stream())
+    gathered = x[source[:count].long() // top]
+    assert torch.equal(side[:count], gathered) and torch.isnan(side[count:].float()).all()
+    act = torch.full((rows * top, N), float("nan"), dtype=torch.bfloat16, device="cuda")
+    _call("gemm_bf16_tcgen05_pair", "mlr_grouped_product_bf16", side.data_ptr(), K, rows, top, w.data_ptr(), w2.data_ptr(), experts, kind, N, K,
+          act.data_ptr(), N, tiles.data_ptr(), n_tiles.data_ptr(), *shape, status.data_ptr(), native.stream())
+    y = torch.full((rows * top, K), float("nan"), device="cuda")
+    _call("gemm_bf16_tcgen05_pair", "mlr_grouped_product_bf16", act.data_ptr(), N, rows, top, down.data_ptr(), None, experts, 0, K, N, y.data_ptr(), K,
+          tiles.data_ptr(), n_tiles.data_ptr(), 0.0, 0.0, 0.0, status.data_ptr(), native.stream())
+    for e, first, n in tiles.tolist():
+        a = gathered[first:first + n].double()
+        want = _gate(a @ w[e].double().T, a @ w2[e].double().T, kind, *shape)
+        assert torch.allclose(act[first:first + n].double(), want, atol=1e-3, rtol=4e-3)
+        assert torch.allclose(y[first:first + n].double(), act[first:first + n].double() @ down[e].double().T, atol=1e-4, rtol=1e-4)
+    assert torch.isnan(act[count:].float()).all() and torch.isnan(y[count:]).all() and status.item() == 0

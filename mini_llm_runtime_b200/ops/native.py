@@ -113,6 +113,11 @@ _SIGNATURES = {
         "mlr_attention_masked_tiles": [c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int,
                                        c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p],
     },
+    "attention_masked_tcgen05": {
+        "mlr_attention_masked_wide_fit": [c_void_p, c_int],
+        "mlr_attention_masked_wide": [c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int,
+                                       c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p],
+    },
     "recurrence": {
         "mlr_linear_recurrence": [c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_longlong, c_void_p,
                                   c_int, c_int, c_void_p, c_void_p, c_void_p],

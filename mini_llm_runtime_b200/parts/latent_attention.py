@@ -90,7 +90,7 @@ class LatentAttentionMixer(Mixer):
         return specs
 
     def kernel_modules(self, dtype) -> List[str]:
-        return ["latent", "attention_masked"] + (["experts"] if dtype is torch.bfloat16 else []) + F.product_modules(dtype)
+        return ["latent", "attention_masked", "attention_masked_tcgen05"] + (["experts"] if dtype is torch.bfloat16 else []) + F.product_modules(dtype)
 
     def _per_head(self, b, x, w, w_t, y, inputs: int, outputs: int, x_step: int, y_step: int) -> None:
         """y[m, h * y_step + :outputs] = x[m, h * x_step + :inputs] W_h: on the tensor cores (the batched product of `experts.cu`) for

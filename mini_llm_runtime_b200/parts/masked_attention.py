@@ -155,7 +155,7 @@ class MaskedAttentionMixer(SequenceCore):
         return self.heads * self.vdim
 
     def kernel_modules(self, dtype) -> List[str]:
-        return ["attention_masked"] + (A.modules_for(dtype, self.dim) if self.dense else []) + F.product_modules(dtype)
+        return ["attention_masked", "attention_masked_tcgen05"] + (A.modules_for(dtype, self.dim) if self.dense else []) + F.product_modules(dtype)
 
     def bind_core(self, tensors, rt, out_scale: float) -> None:
         freq = self.position.frequencies() if self.position is not None else None
@@ -237,8 +237,9 @@ def emit_masked_attention(b, desc: MaskedAttentionSpec, q, gate, act, run: RunCo
                  b.meta("segment_of_row"), table, stride, b.page_size, proj.rows, None, 0, None, 0, 1, 1, None, b.status, b.stream)
         return
     # The step's launch plan (made by the native executor from the step's segments, shared by all layers):
-    # segments of few rows (a decoded token, a short portion) go to the row kernel, prompt portions in tiles of 64
-    # rows to the tensor-core kernel.
+    # segments of few rows (a decoded token, a short portion) go to the row kernel, prompt portions in tiles of 128 rows
+    # to the tcgen05 kernel where it takes the description, a remainder of up to 64 rows and everything else in tiles of 64
+    # rows to the mma.sync kernel.
     # The row kernel cuts long contexts into key ranges that run as blocks of their own (the plan's split of the keys and
     # its scratch for the ranges' partial results: 16 rows x kv heads x splits x (head size + 2) floats per segment).
     # The planner sizes the scratch by the head size it is told: FINER times the room of a range's (value size + 2)
@@ -250,11 +251,16 @@ def emit_masked_attention(b, desc: MaskedAttentionSpec, q, gate, act, run: RunCo
     # ONE row, a decoded token), and sizes the ranges' scratch for them.
     group = heads // kv_heads
     chunks = (group + 15) // 16
-    plan = b.plan((min(group, 16), kv_heads * chunks, 0, 0, finer * (max(dim, vdim) + 2), 1))
+    wide = bool(maps == 1 and getattr(b.rt, "tcgen05_attention", True) and proj.ld % 8 == 0 and act.ld % 8 == 0 and proj.ptr % 16 == 0
+                and act.ptr % 16 == 0 and native.module("attention_masked_tcgen05").mlr_attention_masked_wide_fit(address(desc), b.page_size))
+    plan = b.plan((min(group, 16), kv_heads * chunks, 0, int(wide), finer * (max(dim, vdim) + 2), 1))
     info = b.meta("segment_info")
     split = (plan.chunk, plan.max_splits, finer, plan.scratch)
     b.launch("attention_masked", "mlr_attention_masked", *args, 1, *where, b.meta("positions"), b.meta("segment_of_row"), table,
              stride, b.page_size, 0, plan.items, plan.n_items, info, *split, b.status, b.stream, need=plan.n_items)
+    if wide:
+        b.launch("attention_masked_tcgen05", "mlr_attention_masked_wide", *args, *where, plan.wide_tiles, plan.n_wide, info, table, stride,
+                 b.page_size, b.status, b.stream, need=plan.n_wide)
     b.launch("attention_masked", "mlr_attention_masked_tiles", *args, *where, plan.tiles, plan.n_tiles, info, table, stride,
              b.page_size, b.status, b.stream, need=plan.n_tiles)
 

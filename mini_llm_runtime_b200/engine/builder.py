@@ -184,7 +184,7 @@ class EagerBuilder(_NormHints):
         return len(self.step.segments)
 
     def plan(self, spec: Tuple[int, int, int, int, int, int]) -> PlanRef:
-        """spec: (query heads per kv head, kv heads, window, wide tiles allowed, head size, small allowed)."""
+        """spec: (query heads per kv head, kv heads, window, wide tiles (0 none, 1 where a portion has more than 64 rows, 2 for all), head size, small allowed)."""
         key = ("attention_plan",) + tuple(spec)
         found = self.step.scratch.get(key)
         if found is not None:

@@ -5,8 +5,8 @@ bfloat16, head size a multiple of 16: the tensor-core kernels.  Segments that br
 at most 16 rows per kv head (a decoded token, a portion of two or three tokens) go
 to the split-KV kernel; the rest are prompt portions and go to the flash kernels: with
 head size 64 or 128 (and a page size the kernel takes) in 128-row tiles to the tcgen05
-kernel, a remainder of up to 64 rows and everything else in 64-row tiles to the mma.sync
-kernel.  A mixed step launches all of them.  Other head sizes in bfloat16 use the generic
+kernel when a portion of the step has more than 64 rows, otherwise in 64-row tiles to the
+mma.sync kernel.  Other head sizes in bfloat16 use the generic
 kernel.
 
 The plan (which segments go where, how the keys are split) depends only on the
@@ -80,7 +80,7 @@ def paged_attention(b, qkv, out, cache, group, q_heads, kv_heads, head_dim, wind
              plan.items, plan.n_items, info, table, stride, b.page_size, q_heads, kv_heads, head_dim, int(window), float(scale),
              plan.chunk, plan.max_splits, plan.scratch, plan.counters, b.status, b.stream,
              need=plan.n_items if fresh is None else plan.n_items_beside)
-    # Prompt portions: 128-row tiles on the tcgen05 kernel, the rest in 64-row tiles on the mma.sync kernel.
+    # Prompt portions: in 128-row tiles on the tcgen05 kernel, or in 64-row tiles on the mma.sync kernel.
     if wide:
         b.launch("attention_tcgen05", "mlr_attention_prefill_tcgen05", qkv.ptr, qkv.ld, qkv.rows, out.ptr, out.ld,
                  cache.data_ptr(), cache.shape[0], plan.wide_tiles, plan.n_wide, info, table, stride, b.page_size, q_heads,

@@ -238,8 +238,7 @@ def emit_masked_attention(b, desc: MaskedAttentionSpec, q, gate, act, run: RunCo
         return
     # The step's launch plan (made by the native executor from the step's segments, shared by all layers):
     # segments of few rows (a decoded token, a short portion) go to the row kernel, prompt portions in tiles of 128 rows
-    # to the tcgen05 kernel where it takes the description, a remainder of up to 64 rows and everything else in tiles of 64
-    # rows to the mma.sync kernel.
+    # to the tcgen05 kernel where it takes the description, otherwise in tiles of 64 rows to the mma.sync kernel.
     # The row kernel cuts long contexts into key ranges that run as blocks of their own (the plan's split of the keys and
     # its scratch for the ranges' partial results: 16 rows x kv heads x splits x (head size + 2) floats per segment).
     # The planner sizes the scratch by the head size it is told: FINER times the room of a range's (value size + 2)
@@ -253,7 +252,7 @@ def emit_masked_attention(b, desc: MaskedAttentionSpec, q, gate, act, run: RunCo
     chunks = (group + 15) // 16
     wide = bool(maps == 1 and getattr(b.rt, "tcgen05_attention", True) and proj.ld % 8 == 0 and act.ld % 8 == 0 and proj.ptr % 16 == 0
                 and act.ptr % 16 == 0 and native.module("attention_masked_tcgen05").mlr_attention_masked_wide_fit(address(desc), b.page_size))
-    plan = b.plan((min(group, 16), kv_heads * chunks, 0, int(wide), finer * (max(dim, vdim) + 2), 1))
+    plan = b.plan((min(group, 16), kv_heads * chunks, 0, 2 * int(wide), finer * (max(dim, vdim) + 2), 1))
     info = b.meta("segment_info")
     split = (plan.chunk, plan.max_splits, finer, plan.scratch)
     b.launch("attention_masked", "mlr_attention_masked", *args, 1, *where, b.meta("positions"), b.meta("segment_of_row"), table,

@@ -33,6 +33,7 @@
 // the slot).  Everything but the loads of the projections and the store of the result is float32.
 #include "common.cuh"
 
+#include <algorithm>
 #include <type_traits>
 
 struct RecurrenceSpec {
@@ -644,19 +645,56 @@ __global__ void __launch_bounds__(kScanWarps * 32) recurrence_scan_kernel(const 
         }
 }
 
-// The same walk for head sizes DIM that are a multiple of 32, with sixteen lanes a column: a lane keeps DIM / 16 state values of ONE column,
-// eight warps share the block's 16 columns (two warps a scheduler hide one another's waits).  Four tokens at a time: the sums of their
-// outputs over a column's lanes are exchanged together (five exchanges for four tokens), and nothing is stored to shared memory in
-// between; a token's k, q and decays are loaded from shared memory while the token before it is walked.
-constexpr int kColumnLanes = 16, kColumnWarps = kScanBlockCols * kColumnLanes / 32;
+// Two float32 operations; PACKED: in one instruction (sm_100a).
+template <bool PACKED>
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    if constexpr (!PACKED) return make_float2(fmaf(a.x, b.x, c.x), fmaf(a.y, b.y, c.y));
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;\n"
+        : "=l"(d)
+        : "l"(*reinterpret_cast<unsigned long long*>(&a)), "l"(*reinterpret_cast<unsigned long long*>(&b)),
+          "l"(*reinterpret_cast<unsigned long long*>(&c)));
+    return *reinterpret_cast<float2*>(&d);
+}
+template <bool PACKED>
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+    if constexpr (!PACKED) return make_float2(a.x * b.x, a.y * b.y);
+    unsigned long long d;
+    asm("mul.rn.f32x2 %0, %1, %2;\n" : "=l"(d) : "l"(*reinterpret_cast<unsigned long long*>(&a)), "l"(*reinterpret_cast<unsigned long long*>(&b)));
+    return *reinterpret_cast<float2*>(&d);
+}
+
+// The same walk for head sizes DIM that are a multiple of 32, with L lanes a column: a lane keeps DIM / L state values of ONE column, the
+// block's 16 columns take L / 2 warps.  Four tokens at a time: the sums of their outputs over a column's lanes are exchanged together
+// (four or five exchanges for four tokens), and nothing is stored to shared memory in between; a token's k, q and decays are loaded
+// from shared memory while the token before it is walked.  It is bound by the waits of one or two warps a scheduler for one another's
+// results (an instruction every five cycles a warp), hence the packed operations and, for the delta and step rules, eight lanes a
+// column instead of sixteen (loads of k and q serve twice the columns, one exchange less): 2048 and 900 tokens of 16 heads of
+// 128 x 128 with the delta rule and channel decays 623 -> 548 us, 2048 tokens with one decay a head 400 -> 352 us, 1999 tokens of 128
+// heads of 128 x 64 with the step rule 577 -> 458 us.
+// Neither helps the decay rule (gated linear attention of those sizes: 430 to 510 us either way), nor two delta tokens at once.
+__host__ __device__ constexpr int column_lanes(int dim, int rule) { return rule != 0 && dim <= 128 ? 8 : 16; }
+__host__ __device__ constexpr int column_warps(int dim, int rule) { return kScanBlockCols * column_lanes(dim, rule) / 32; }
+
+// PASS: 0 walks a segment whole.  The decay and step rules can walk it in pieces that run side by side, since what a piece makes of the
+// state before it is a product with its decays: pass 1 walks the first piece as it is and the others but the last from a state
+// of zero, without outputs, and leaves their ends and the products of their decays in `ends`; pass 2 puts the state before each later
+// piece together from those and walks the piece.  The walk of one request's 2048 tokens over 8 heads has 64 blocks for 148 SMs and every
+// token waits for the one before: 2048 rows 270 us whole, 60 + 90 us in 16 pieces.
+constexpr int kLeastPiece = 128;          // tokens of a piece at least: `ends` has a place for every 128 rows
+struct WalkPieces {
+    float* ends;                          // [rows / 128][heads][(vdim + 1)][dim]: a piece's end by column, then its decays' products
+    int most;                             // pieces of a segment
+};
+__host__ __device__ inline size_t ends_of_piece(const RecurrenceSpec& s) { return static_cast<size_t>(s.heads) * (s.vdim + 1) * s.dim; }
 
 // NC: columns of the state a lane works on (column c and c + 16): two halve the reading of k and q where blocks outnumber the SMs.
-template <typename T, int DIM, int RULE, bool CH, int NC>
-__global__ void __launch_bounds__(kColumnWarps * 32) recurrence_scan16_kernel(const float* qf, const float* kf, const float* df, const float* gates,
+template <typename T, int DIM, int RULE, bool CH, int NC, int PASS>
+__global__ void __launch_bounds__(column_warps(DIM, RULE) * 32) recurrence_scan16_kernel(const float* qf, const float* kf, const float* df, const float* gates,
                                                                             const T* proj, int ld, float* obuf, float* state, long long state_stride,
-                                                                            const int* segment_info, RecurrenceSpec s, int batch) {
+                                                                            const int* segment_info, RecurrenceSpec s, int batch, WalkPieces pieces) {
     mlr_grid_wait();
-    constexpr int kThreads = kColumnWarps * 32, E = DIM / kColumnLanes, V = E % 4 == 0 ? 4 : 2;       // V: values an access
+    constexpr int kColumnLanes = column_lanes(DIM, RULE), kThreads = column_warps(DIM, RULE) * 32, E = DIM / kColumnLanes, V = E % 4 == 0 ? 4 : 2;       // V: values an access
     constexpr int kCols = kScanBlockCols * NC;
     extern __shared__ __align__(16) unsigned char smem[];
     const int stage = batch * DIM;                             // batch: a multiple of 4, at most 32
@@ -667,8 +705,22 @@ __global__ void __launch_bounds__(kColumnWarps * 32) recurrence_scan16_kernel(co
     float* os = vs + batch * kCols;                   // [batch][kCols]
     float* gs = os + batch * kCols;                   // [batch]
     float* bs = gs + batch;                                    // [batch]
-    const int segment = blockIdx.x, head = blockIdx.y, block_col = blockIdx.z * kCols;
-    const int first = segment_info[4 * segment], count = segment_info[4 * segment + 1], slot = segment_info[4 * segment + 3];
+    const int segment = PASS ? blockIdx.x / pieces.most : blockIdx.x, head = blockIdx.y, block_col = blockIdx.z * kCols;
+    int first = segment_info[4 * segment], count = segment_info[4 * segment + 1];
+    const int slot = segment_info[4 * segment + 3];
+    int piece = 0, piece_rows = count;
+    bool last = true;                     // of the segment's pieces: its end is the segment's
+    const int segment_first = first;
+    if (PASS) {
+        piece = blockIdx.x % pieces.most;
+        piece_rows = max(kLeastPiece, ((count + pieces.most - 1) / pieces.most + 3) / 4 * 4);
+        const int n = (count + piece_rows - 1) / piece_rows;
+        last = piece == n - 1;
+        if (piece >= n || (PASS == 1 ? piece > 0 && last : piece == 0)) return;
+        first += piece * piece_rows;
+        count = min(piece_rows, count - piece * piece_rows);
+    }
+    const bool with_outputs = PASS != 1 || piece == 0;
     const int qk_head = head / (s.heads / s.qk_heads);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int sub = lane & (kColumnLanes - 1), my_col = warp * (32 / kColumnLanes) + lane / kColumnLanes;
@@ -676,15 +728,45 @@ __global__ void __launch_bounds__(kColumnWarps * 32) recurrence_scan16_kernel(co
     const size_t o_ld = static_cast<size_t>(s.heads) * s.vdim;
     const float decay = !CH && RULE == 0 ? s.decay[head] : 1.0f;
 
-    float S[NC][E];
+    constexpr int H = E / 2;              // pairs of values
+    constexpr bool P = RULE != 0;         // packed
+    float2 S[NC][H];
     float* my_state = state + static_cast<size_t>(slot) * state_stride + (static_cast<size_t>(head) * s.vdim + block_col + my_col) * DIM;
     auto live = [&](int n) { return block_col + my_col + n * kScanBlockCols < s.vdim; };
-    // Value j of a lane is value V * (16 * (j / V) + sub) + j % V of the head: sixteen lanes read consecutive bytes.
+    // Value j of a lane is value V * (L * (j / V) + sub) + j % V of the head: a column's lanes read consecutive bytes.
     auto place = [&](int j) { return V * (kColumnLanes * (j / V) + sub) + j % V; };
+    auto pair_at = [](const float* p) { return make_float2(p[0], p[1]); };       // (a slot of the state may start anywhere)
+    auto twice = [](float x) { return make_float2(x, x); };
+    auto whole = [](float2 a) { return a.x + a.y; };
 #pragma unroll
     for (int n = 0; n < NC; ++n)
 #pragma unroll
-        for (int j = 0; j < E; ++j) S[n][j] = live(n) ? my_state[n * kScanBlockCols * DIM + place(j)] : 0.0f;
+        for (int j = 0; j < H; ++j) S[n][j] = live(n) && piece == 0 ? pair_at(my_state + n * kScanBlockCols * DIM + place(2 * j)) : twice(0.0f);
+    // The end of a piece for this lane's columns, and the products of its decays.
+    auto end_of = [&](int piece_first) {
+        return pieces.ends + piece_first / kLeastPiece * ends_of_piece(s) + (static_cast<size_t>(head) * (s.vdim + 1) + block_col + my_col) * DIM;
+    };
+    auto decays_of = [&](int piece_first) {
+        return pieces.ends + piece_first / kLeastPiece * ends_of_piece(s) + (static_cast<size_t>(head) * (s.vdim + 1) + s.vdim) * DIM;
+    };
+    if (PASS == 2) {
+        for (int before = 0; before < piece; ++before) {
+            const float* end = end_of(segment_first + before * piece_rows);
+            const float* d = decays_of(segment_first + before * piece_rows);
+#pragma unroll
+            for (int j = 0; j < H; ++j) {
+                const float2 decayed = before > 0 ? __ldcg(reinterpret_cast<const float2*>(d + place(2 * j))) : twice(0.0f);      // nothing lies before the first piece
+#pragma unroll
+                for (int n = 0; n < NC; ++n)
+                    if (live(n)) S[n][j] = fma2<P>(decayed, S[n][j], __ldcg(reinterpret_cast<const float2*>(end + n * kScanBlockCols * DIM + place(2 * j))));
+            }
+        }
+    }
+    // The lanes of one warp of a head keep the products of the decays of their values.
+    const bool track = PASS == 1 && blockIdx.z == 0 && warp == 0;
+    float2 product[PASS == 1 ? H : 1];
+#pragma unroll
+    for (int j = 0; j < (PASS == 1 ? H : 1); ++j) product[j] = twice(1.0f);
 
     constexpr int kVPerThread = 32 * kCols / kThreads;
     T v_next[kVPerThread];                // as loaded: a conversion right behind the load would wait for it
@@ -701,7 +783,7 @@ __global__ void __launch_bounds__(kColumnWarps * 32) recurrence_scan16_kernel(co
         constexpr int kPerRow = DIM / 4;
         for (int i = threadIdx.x; i < n * kPerRow; i += kThreads) {
             const int t = i / kPerRow, c = (i % kPerRow) * 4;
-            mlr_async_copy16(qdst + t * DIM + c, qsrc + t * qk_ld + c);
+            if (with_outputs) mlr_async_copy16(qdst + t * DIM + c, qsrc + t * qk_ld + c);
             mlr_async_copy16(kdst + t * DIM + c, ksrc + t * qk_ld + c);
             if constexpr (CH) mlr_async_copy16(ddst + t * DIM + c, dsrc + t * d_ld + c);
         }
@@ -720,7 +802,7 @@ __global__ void __launch_bounds__(kColumnWarps * 32) recurrence_scan16_kernel(co
     };
 
     struct Token {
-        float k[E], q[E], d[CH ? E : 1];
+        float2 k[H], q[H], d[CH ? H : 1];
     };
     fetch(0, 0);
     int current = 0;
@@ -742,28 +824,28 @@ __global__ void __launch_bounds__(kColumnWarps * 32) recurrence_scan16_kernel(co
         const float* qnow = qs + current * stage + V * sub;
         const float* know = ks + current * stage + V * sub;
         const float* dnow = ds + current * stage + V * sub;
-        auto load = [&](Token& x, int t) {
-            auto vector = [&](float* into, const float* from) {
+        auto load = [&](Token& x, int t, bool with_q) {
+            auto vector = [&](float2* into, const float* from) {
 #pragma unroll
                 for (int e = 0; e < E / V; ++e) {
                     if constexpr (V == 4) {
                         const float4 y = *reinterpret_cast<const float4*>(from + t * DIM + V * kColumnLanes * e);
-                        into[4 * e] = y.x; into[4 * e + 1] = y.y; into[4 * e + 2] = y.z; into[4 * e + 3] = y.w;
+                        into[2 * e] = make_float2(y.x, y.y);
+                        into[2 * e + 1] = make_float2(y.z, y.w);
                     } else {
-                        const float2 y = *reinterpret_cast<const float2*>(from + t * DIM + V * kColumnLanes * e);
-                        into[2 * e] = y.x; into[2 * e + 1] = y.y;
+                        into[e] = *reinterpret_cast<const float2*>(from + t * DIM + V * kColumnLanes * e);
                     }
                 }
             };
             vector(x.k, know);
             if constexpr (CH) vector(x.d, dnow);
-            vector(x.q, qnow);
+            if (with_q) vector(x.q, qnow);
         };
         Token tokens[2];
-        load(tokens[0], 0);
+        load(tokens[0], 0, with_outputs);
         // GUARDED: the batch's last, incomplete group of four.  Rows past the batch are not read: a token's successor is at most the last.
-        auto walk4 = [&](int t0, auto guarded) {
-            constexpr bool kGuarded = decltype(guarded)::value;
+        auto walk4 = [&](int t0, auto guarded, auto outputs) {
+            constexpr bool kGuarded = decltype(guarded)::value, kOutputs = decltype(outputs)::value;
             float v[NC][4];
 #pragma unroll
             for (int m = 0; m < NC; ++m) {
@@ -786,34 +868,44 @@ __global__ void __launch_bounds__(kColumnWarps * 32) recurrence_scan16_kernel(co
                 for (int m = 0; m < NC; ++m) dots[m][u] = 0.0f;
                 if (!kGuarded || t0 + u < n) {
                     const Token& x = tokens[u & 1];
-                    load(tokens[(u + 1) & 1], u < 3 && !kGuarded ? t0 + u + 1 : min(t0 + u + 1, n - 1));
+                    load(tokens[(u + 1) & 1], u < 3 && !kGuarded ? t0 + u + 1 : min(t0 + u + 1, n - 1), kOutputs);
 #pragma unroll
                     for (int m = 0; m < NC; ++m) {
                         float write = RULE == 2 ? beta[u] * v[m][u] : v[m][u];
+                        auto decay_at = [&](int j) { return CH ? x.d[CH ? j : 0] : twice(g[u]); };
                         if constexpr (RULE != 1) {
 #pragma unroll
-                            for (int j = 0; j < E; ++j) S[m][j] = fmaf(CH ? x.d[CH ? j : 0] : g[u], S[m][j], x.k[j] * write);
+                            for (int j = 0; j < H; ++j) S[m][j] = fma2<P>(decay_at(j), S[m][j], mul2<P>(x.k[j], twice(write)));
                         } else {
-                            float c[2] = {};
+                            float2 c[2] = {};
 #pragma unroll
-                            for (int j = 0; j < E; ++j) {
-                                S[m][j] *= CH ? x.d[CH ? j : 0] : g[u];
-                                c[j & 1] = fmaf(S[m][j], x.k[j], c[j & 1]);
+                            for (int j = 0; j < H; ++j) {
+                                S[m][j] = mul2<P>(S[m][j], decay_at(j));
+                                c[j & 1] = fma2<P>(S[m][j], x.k[j], c[j & 1]);
                             }
-                            float held = c[0] + c[1];
+                            float held = whole(c[0]) + whole(c[1]);
 #pragma unroll
                             for (int step = 1; step < kColumnLanes; step *= 2) held += __shfl_xor_sync(0xffffffffu, held, step);
                             write = beta[u] * (write - held);
 #pragma unroll
-                            for (int j = 0; j < E; ++j) S[m][j] = fmaf(x.k[j], write, S[m][j]);
+                            for (int j = 0; j < H; ++j) S[m][j] = fma2<P>(x.k[j], twice(write), S[m][j]);
                         }
-                        float o[2] = {};
+                        if constexpr (kOutputs) {
+                            float2 o[2] = {};
 #pragma unroll
-                        for (int j = 0; j < E; ++j) o[j & 1] = fmaf(S[m][j], x.q[j], o[j & 1]);
-                        dots[m][u] = o[0] + o[1];
+                            for (int j = 0; j < H; ++j) o[j & 1] = fma2<P>(S[m][j], x.q[j], o[j & 1]);
+                            dots[m][u] = whole(o[0]) + whole(o[1]);
+                        }
+                    }
+                    if constexpr (PASS == 1 && !kOutputs) {
+                        if (track) {
+#pragma unroll
+                            for (int j = 0; j < H; ++j) product[j] = mul2<P>(product[j], CH ? x.d[CH ? j : 0] : twice(g[u]));
+                        }
                     }
                 }
             }
+            if constexpr (!kOutputs) return;
             // Lanes with sub % 4 == u end up with the sum of token t0 + u.
             const bool odd = sub & 1, high = sub & 2;
 #pragma unroll
@@ -821,15 +913,23 @@ __global__ void __launch_bounds__(kColumnWarps * 32) recurrence_scan16_kernel(co
                 const float even_pair = (odd ? dots[m][1] : dots[m][0]) + __shfl_xor_sync(0xffffffffu, odd ? dots[m][0] : dots[m][1], 1);
                 const float odd_pair = (odd ? dots[m][3] : dots[m][2]) + __shfl_xor_sync(0xffffffffu, odd ? dots[m][2] : dots[m][3], 1);
                 float sum = (high ? odd_pair : even_pair) + __shfl_xor_sync(0xffffffffu, high ? even_pair : odd_pair, 2);
-                sum += __shfl_xor_sync(0xffffffffu, sum, 4);
-                sum += __shfl_xor_sync(0xffffffffu, sum, 8);
+#pragma unroll
+                for (int step = 4; step < kColumnLanes; step *= 2) sum += __shfl_xor_sync(0xffffffffu, sum, step);
                 if (sub < 4 && (!kGuarded || t0 + sub < n)) os[(t0 + sub) * kCols + my_col + m * kScanBlockCols] = sum;
             }
         };
         for (int t0 = 0; t0 < n; t0 += 4) {
-            if (t0 + 4 <= n) walk4(t0, std::false_type{});      // whole groups carry no per-token conditions
-            else walk4(t0, std::true_type{});
+            if constexpr (PASS == 1) {
+                if (!with_outputs) {
+                    if (t0 + 4 <= n) walk4(t0, std::false_type{}, std::false_type{});
+                    else walk4(t0, std::true_type{}, std::false_type{});
+                    continue;
+                }
+            }
+            if (t0 + 4 <= n) walk4(t0, std::false_type{}, std::true_type{});      // whole groups carry no per-token conditions
+            else walk4(t0, std::true_type{}, std::true_type{});
         }
+        if (!with_outputs) continue;
         __syncthreads();
         for (int i = threadIdx.x; i < n * kCols; i += kThreads) {
             const int t = i / kCols, c = block_col + i % kCols;
@@ -838,12 +938,21 @@ __global__ void __launch_bounds__(kColumnWarps * 32) recurrence_scan16_kernel(co
         }
     }
     mlr_grid_dependents_may_start();     // only now: blocks of the next grid that wait on this SM slow the walk
+    float* to = last ? my_state : end_of(first);
 #pragma unroll
     for (int n = 0; n < NC; ++n)
         if (live(n)) {
 #pragma unroll
-            for (int j = 0; j < E; ++j) my_state[n * kScanBlockCols * DIM + place(j)] = S[n][j];
+            for (int j = 0; j < H; ++j) {
+                float* cell = to + n * kScanBlockCols * DIM + place(2 * j);
+                cell[0] = S[n][j].x;
+                cell[1] = S[n][j].y;
+            }
         }
+    if (track && !last && lane < kColumnLanes) {
+#pragma unroll
+        for (int j = 0; j < H; ++j) *reinterpret_cast<float2*>(decays_of(first) + place(2 * j)) = product[PASS == 1 ? j : 0];
+    }
 }
 
 
@@ -1084,10 +1193,11 @@ MLR_API int mlr_linear_recurrence(const RecurrenceSpec* spec, const void* proj, 
 // obuf: float32 [rows, heads * vdim].  Same results as `mlr_linear_recurrence` up to the order in which a column's sums are added
 // (the same order for head sizes that are no multiple of 32).  With a decay per channel, df [rows, heads * dim] and (low-rank gate) gf
 // [rows, heads * vdim] are float32 room; with `products_made` they hold the low-rank products' results already (df without the bias).
-MLR_API int mlr_linear_recurrence_split(const RecurrenceSpec* spec, const void* proj, int ld, const void* side, int ld_side, int act_bf16,
-                                        void* out, int ld_out, float* state, long long state_stride, const int* segment_info,
-                                        int n_segments, const int* positions, int rows, float* qf, float* kf, float* gates, float* obuf,
-                                        float* df, float* gf, int products_made, cudaStream_t stream) {
+// ends: float32 room for the ends of a walk's pieces, rows / 128 times heads * (vdim + 1) * dim values, or null (segments are walked whole).
+MLR_API int mlr_linear_recurrence_pieces(const RecurrenceSpec* spec, const void* proj, int ld, const void* side, int ld_side, int act_bf16,
+                                         void* out, int ld_out, float* state, long long state_stride, const int* segment_info,
+                                         int n_segments, const int* positions, int rows, float* qf, float* kf, float* gates, float* obuf,
+                                         float* df, float* gf, int products_made, float* ends, cudaStream_t stream) {
     MLR_REQUIRE(spec, "linear_recurrence_split: no description");
     const RecurrenceSpec& s = *spec;
     if (check_recurrence(s)) return 1;
@@ -1104,7 +1214,7 @@ MLR_API int mlr_linear_recurrence_split(const RecurrenceSpec* spec, const void* 
     const bool two = s.rule == 2 && fixed_size && column_blocks > 1 && static_cast<long long>(n_segments) * s.heads * column_blocks > mlr_sm_count();
     const int block_cols = kScanBlockCols * (two ? 2 : 1);
     const size_t per_token = sizeof(float) * ((channel ? 6 : 4) * static_cast<size_t>(s.dim) + 2 * block_cols + 2);
-    int batch = static_cast<int>(((channel ? 84 : 44) * 1024) / per_token);
+    int batch = static_cast<int>(((channel ? 84 : 72) * 1024) / per_token);
     batch = batch < 1 ? 1 : (batch > 32 ? 32 : batch);
     if (batch > 4) batch -= batch % 4;
     const size_t shared = per_token * batch + (channel ? 16 : 0);
@@ -1114,18 +1224,44 @@ MLR_API int mlr_linear_recurrence_split(const RecurrenceSpec* spec, const void* 
     const dim3 channel_grid((rows + kChannelRows - 1) / kChannelRows,
                             (s.heads * s.dim + per_block - 1) / per_block + (s.gate_rank ? (s.heads * s.vdim + per_block - 1) / per_block : 0));
     const size_t channel_shared = sizeof(float) * kChannelRows * (static_cast<size_t>(s.decay_rank > s.gate_rank ? s.decay_rank : s.gate_rank) + per_block);
+    // Pieces where whole segments leave the SMs short of blocks: up to eight blocks an SM, and at least six pieces (the two passes take
+    // the time of two pieces, and pieces slow one another).  Measured at 2048 rows of 128 x 128: 64 blocks in 16 pieces 270 -> 150 us,
+    // 128 blocks (two requests) in 9 pieces 281 -> 235 us; 256 blocks in 4 pieces 433 -> 580 us.
+    WalkPieces pieces = {ends, 1};
+    if (ends && s.rule != 1 && fixed_size) {
+        const long long blocks = static_cast<long long>(n_segments) * grid.y * grid.z;
+        const long long most = std::min(std::min(8ll * mlr_sm_count() / blocks, static_cast<long long>(rows / n_segments / kLeastPiece)), 16ll);
+        if (most >= 6) pieces.most = static_cast<int>(most);
+    }
+#define MLR_PASS(T, DIM, RULE, CH, NC, PASS)                                                                                           \
+    do {                                                                                                                               \
+        const auto kernel = recurrence_scan16_kernel<T, DIM, RULE, CH, NC, PASS>;                                                      \
+        if (shared > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(shared));   \
+        mlr_launch(kernel, dim3(grid.x * (PASS ? pieces.most : 1), grid.y, grid.z), dim3(column_warps(DIM, RULE) * 32), shared, stream, qf, kf, \
+                   static_cast<const float*>(df), gates, static_cast<const T*>(proj), ld, obuf, state, state_stride, segment_info, s, batch, \
+                   pieces);                                                                                                            \
+    } while (0)
+#define MLR_PASSES(T, DIM, RULE, CH, NC)              \
+    do {                                              \
+        if (pieces.most > 1) {                        \
+            MLR_PASS(T, DIM, RULE, CH, NC, 1);        \
+            MLR_PASS(T, DIM, RULE, CH, NC, 2);        \
+        } else {                                      \
+            MLR_PASS(T, DIM, RULE, CH, NC, 0);        \
+        }                                             \
+    } while (0)
 #define MLR_WALK(KERNEL, T, WARPS)                                                                                                     \
     do {                                                                                                                               \
         if (shared > 48 * 1024) cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(shared));   \
         mlr_launch((KERNEL), dim3(grid), dim3((WARPS) * 32), shared, stream, qf, kf, static_cast<const float*>(df), gates,             \
                    static_cast<const T*>(proj), ld, obuf, state, state_stride, segment_info, s, batch);                                \
     } while (0)
-#define MLR_COLUMN(T, DIM, CH)                                                                                                         \
-    do {                                                                                                                               \
-        if (s.rule == 0) MLR_WALK((recurrence_scan16_kernel<T, DIM, 0, CH, 1>), T, kColumnWarps);                                      \
-        else if (s.rule == 2 && two) MLR_WALK((recurrence_scan16_kernel<T, DIM, 2, false, 2>), T, kColumnWarps);                       \
-        else if (s.rule == 2) MLR_WALK((recurrence_scan16_kernel<T, DIM, 2, false, 1>), T, kColumnWarps);                              \
-        else MLR_WALK((recurrence_scan16_kernel<T, DIM, 1, CH, 1>), T, kColumnWarps);                                                  \
+#define MLR_COLUMN(T, DIM, CH)                                            \
+    do {                                                                  \
+        if (s.rule == 0) MLR_PASSES(T, DIM, 0, CH, 1);                    \
+        else if (s.rule == 2 && two) MLR_PASSES(T, DIM, 2, false, 2);     \
+        else if (s.rule == 2) MLR_PASSES(T, DIM, 2, false, 1);            \
+        else MLR_PASS(T, DIM, 1, CH, 1, 0);                               \
     } while (0)
 #define MLR_SCAN(T, CH)                                                                                                                \
     do {                                                                                                                               \
@@ -1166,5 +1302,15 @@ MLR_API int mlr_linear_recurrence_split(const RecurrenceSpec* spec, const void* 
 #undef MLR_SCAN
 #undef MLR_COLUMN
 #undef MLR_WALK
+#undef MLR_PASSES
+#undef MLR_PASS
     return mlr_launched("linear_recurrence_split");
+}
+
+MLR_API int mlr_linear_recurrence_split(const RecurrenceSpec* spec, const void* proj, int ld, const void* side, int ld_side, int act_bf16,
+                                        void* out, int ld_out, float* state, long long state_stride, const int* segment_info,
+                                        int n_segments, const int* positions, int rows, float* qf, float* kf, float* gates, float* obuf,
+                                        float* df, float* gf, int products_made, cudaStream_t stream) {
+    return mlr_linear_recurrence_pieces(spec, proj, ld, side, ld_side, act_bf16, out, ld_out, state, state_stride, segment_info, n_segments, positions,
+                                        rows, qf, kf, gates, obuf, df, gf, products_made, nullptr, stream);
 }

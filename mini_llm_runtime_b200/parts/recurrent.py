@@ -58,9 +58,11 @@ def emit_recurrence(b, mixer, proj, side, act, run: RunContext) -> None:
     kf = b.temp(proj.rows, d.qk_heads * d.dim, torch.float32)
     gates = b.temp(proj.rows, 2 * d.heads, torch.float32)
     obuf = b.temp(proj.rows, d.heads * d.vdim, torch.float32)
-    b.launch("recurrence", "mlr_linear_recurrence_split", address(d), proj.ptr, proj.ld, side.ptr, side.ld, proj.is_bf16, act.ptr,
+    # Room for the ends of a walk's pieces (a place per 128 rows): rules whose pieces can run side by side.
+    ends = b.temp(proj.rows, -(-d.heads * (d.vdim + 1) * d.dim // 128), torch.float32) if d.rule != 1 else None
+    b.launch("recurrence", "mlr_linear_recurrence_pieces", address(d), proj.ptr, proj.ld, side.ptr, side.ld, proj.is_bf16, act.ptr,
              act.ld, state.data_ptr(), state.stride(0), info, b.segments, b.meta("positions"), proj.rows, qf.ptr, kf.ptr, gates.ptr,
-             obuf.ptr, df.ptr if df else None, gf.ptr if gf else None, made, b.stream)
+             obuf.ptr, df.ptr if df else None, gf.ptr if gf else None, made, ends.ptr if ends else None, b.stream)
 
 
 def emit_short_conv(b, x, taps_weight: torch.Tensor, bias: Optional[torch.Tensor], state: torch.Tensor, state_offset: int):

@@ -94,27 +94,30 @@ __global__ void rmsnorm_kernel(float* __restrict__ h, const float* __restrict__ 
     }
 }
 
-// The same for widths that are multiples of 4 and fit 16 values per thread: each thread
-// keeps its values in registers between the two passes, so the row is read once and every
-// load of the row is in flight at the same time.  One block per row.
-template <typename T, typename W>
+// The same for widths that are multiples of 4 and fit 16 values per thread of the `owners` (a power of two of threads that depends
+// on the width alone): values stay in registers between the two passes, so the row is read once and every load of the
+// row is in flight at the same time.  One block per row.  QUADS 4: a block is the owners, a thread loads its four groups of
+// four values; QUADS 1: four threads stand for an owner.  The sums are the same: four values in a chain, an owner's four
+// groups as (0 + 1) + (2 + 3), then a fixed tree over the owners.
+template <typename T, typename W, int QUADS>
 __global__ void __launch_bounds__(1024) rmsnorm_cached_kernel(float* __restrict__ h, const float* __restrict__ delta,
                                                              int slices, size_t slice_stride,
                                                              const W* __restrict__ weight, T* __restrict__ out,
                                                              const int* __restrict__ rows, int width, float eps,
-                                                             int write_back) {
+                                                             int write_back, int owners) {
     mlr_grid_dependents_may_start();
     mlr_grid_wait();
     __shared__ float scratch[32];
+    __shared__ float groups[QUADS == 1 ? 1024 : 1];
     const int r = blockIdx.x;
     const size_t row = rows ? static_cast<size_t>(rows[r]) : static_cast<size_t>(r);
     float4* hr = reinterpret_cast<float4*>(h + row * width);
     const float4* dr = delta ? reinterpret_cast<const float4*>(delta + row * width) : nullptr;
     const int quads = width >> 2;
-    float4 x[4];
-    float sum = 0.0f;
+    float4 x[QUADS];
+    float sums[QUADS];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
+    for (int k = 0; k < QUADS; ++k) {
         const int i = threadIdx.x + k * blockDim.x;
         x[k] = make_float4(0.f, 0.f, 0.f, 0.f);
         if (i < quads) {
@@ -129,20 +132,28 @@ __global__ void __launch_bounds__(1024) rmsnorm_cached_kernel(float* __restrict_
             }
         }
     }
-    // A fixed order of summation per thread, then a fixed tree over the block: the result
-    // depends on the width alone, not on how many rows the launch has.
+    // A fixed order of summation: the result depends on the width alone, not on how many rows the launch has.
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        sum = fmaf(x[k].x, x[k].x, sum);
-        sum = fmaf(x[k].y, x[k].y, sum);
-        sum = fmaf(x[k].z, x[k].z, sum);
-        sum = fmaf(x[k].w, x[k].w, sum);
+    for (int k = 0; k < QUADS; ++k) sums[k] = fmaf(x[k].w, x[k].w, fmaf(x[k].z, x[k].z, fmaf(x[k].y, x[k].y, x[k].x * x[k].x)));
+    float sum;
+    if constexpr (QUADS == 1) {
+        groups[threadIdx.x] = sums[0];
+        __syncthreads();
+        const int owner = threadIdx.x & (owners - 1);
+        sum = (groups[owner] + groups[owner + owners]) + (groups[owner + 2 * owners] + groups[owner + 3 * owners]);
+    } else {
+        sum = (sums[0] + sums[1]) + (sums[2 % QUADS] + sums[3 % QUADS]);
     }
-    sum = mlr_block_sum(sum, scratch);
+    // The owners' sums once each: by the first owners' warps, whichever QUADS.
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = owners >> 5;
+    sum = mlr_warp_sum(sum);
+    if (lane == 0 && warp < warps) scratch[warp] = sum;
+    __syncthreads();
+    sum = mlr_warp_sum(lane < warps ? scratch[lane] : 0.0f);
     const float scale = 1.0f / sqrtf(sum / static_cast<float>(width) + eps);
     T* dst = out + static_cast<size_t>(r) * width;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
+    for (int k = 0; k < QUADS; ++k) {
         const int i = threadIdx.x + k * blockDim.x;
         if (i < quads) {
             if (write_back && dr) hr[i] = x[k];
@@ -541,21 +552,24 @@ MLR_API int mlr_rmsnorm(float* h, const float* delta, int slices, long long slic
     if (count == 0) return 0;
     const int threads = row_threads(width);
     // Register-cached path: width a multiple of 4, at most 16 values per thread of a block
-    // of up to 1024 threads, 16-byte aligned rows.  A thread takes 16 values where the width allows: its four loads are
-    // on their way together and several blocks share an SM.  With four values a thread a row of 4096 was one block of 1024
-    // threads an SM (registers), which waited for memory and for its own sum with nothing beside it: 2048 rows of 4096
-    // 34 us, with 256 threads a row 14 us.
+    // of up to 1024 threads, 16-byte aligned rows.  A thread takes 16 values where the rows outnumber the SMs: its four loads are
+    // on their way together and several blocks share an SM.  With four values a thread a row of 4096 is one block of 1024
+    // threads an SM (registers), which waits for memory and for its own sum with nothing beside it: 2048 rows of 4096
+    // 34 us, with 256 threads a row 14 us.  Rows that have an SM each are better off with more threads (the 8B decode step of 40
+    // rows: 5.51 ms with 256 threads a row, 5.40 ms with 1024).
     int cached_threads = 64;
     while (cached_threads < 1024 && cached_threads * 16 < width) cached_threads <<= 1;
+    const bool spread = cached_threads <= 256 && count <= mlr_sm_count();
     const bool cached = width % 4 == 0 && width <= cached_threads * 16 && reinterpret_cast<uintptr_t>(h) % 16 == 0 &&
                         (!delta || (reinterpret_cast<uintptr_t>(delta) % 16 == 0 && slice_stride % 4 == 0)) &&
                         reinterpret_cast<uintptr_t>(out) % 16 == 0 && reinterpret_cast<uintptr_t>(weight) % 16 == 0;
 #define MLR_LAUNCH(T, W)                                                                                   \
     do {                                                                                                   \
         if (cached)                                                                                        \
-            mlr_launch((rmsnorm_cached_kernel<T, W>), dim3(count), dim3(cached_threads), 0, stream,                              \
+            mlr_launch((spread ? rmsnorm_cached_kernel<T, W, 1> : rmsnorm_cached_kernel<T, W, 4>), dim3(count), \
+                dim3(spread ? 4 * cached_threads : cached_threads), 0, stream,                             \
                 h, delta, slices, static_cast<size_t>(slice_stride), static_cast<const W*>(weight),       \
-                static_cast<T*>(out), rows, width, eps, write_back);                                       \
+                static_cast<T*>(out), rows, width, eps, write_back, cached_threads);                       \
         else                                                                                               \
             mlr_launch((rmsnorm_kernel<T, W>), dim3(count), dim3(threads), 0, stream, h, delta, slices, static_cast<size_t>(slice_stride), \
                                                                  static_cast<const W*>(weight),            \

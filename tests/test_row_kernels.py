@@ -40,6 +40,11 @@ def test_rms_norm(dtype, width):
     _call("elementwise", "mlr_rmsnorm", h.data_ptr(), None, 1, 0, weight.data_ptr(), 0, out.data_ptr(), native.is_bf16(out), None, rows, width, 1e-5, 0,
           native.stream())
     _near(out, _grouped(h.double(), 1, 1e-5) * weight.double(), dtype)
+    # Many rows, which take fewer threads each, give the same bits.
+    many, all_out = h.repeat(200, 1), torch.empty(200 * rows, width, dtype=dtype, device="cuda")
+    _call("elementwise", "mlr_rmsnorm", many.data_ptr(), None, 1, 0, weight.data_ptr(), 0, all_out.data_ptr(), native.is_bf16(out), None, 200 * rows, width,
+          1e-5, 0, native.stream())
+    assert torch.equal(all_out, out.repeat(200, 1))
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])

@@ -79,49 +79,72 @@ __global__ void __launch_bounds__(kRouteThreads) route_kernel(const T* x, long l
 #pragma unroll
     for (int r = 0; r < ROWS; ++r) {
         const T* xrow = x + static_cast<size_t>(min(row0 + r, rows - 1)) * ld;
-        for (int c = threadIdx.x; c < width; c += blockDim.x) xs[static_cast<size_t>(r) * width + c] = mlr_load(xrow, c);
+        if (width % 4 == 0 && ld % 4 == 0 && reinterpret_cast<uintptr_t>(x) % (4 * sizeof(T)) == 0) {
+            for (int c = threadIdx.x * 4; c < width; c += blockDim.x * 4) {
+                float v[4];
+                mlr_load4(xrow + c, v);
+                *reinterpret_cast<float4*>(xs + static_cast<size_t>(r) * width + c) = make_float4(v[0], v[1], v[2], v[3]);
+            }
+        } else {
+            for (int c = threadIdx.x; c < width; c += blockDim.x) xs[static_cast<size_t>(r) * width + c] = mlr_load(xrow, c);
+        }
     }
     __syncthreads();
-    for (int e = warp; e < experts + has_gate; e += warps) {
-        const float* w = router + static_cast<size_t>(e) * width;
-        float sums[ROWS] = {};
+    // With four tokens a block a warp takes two experts at a time: what it reads of the tokens from shared memory, which bounds it, serves
+    // both: 1999 rows of 4096 and 20 outputs 93 -> 72 us, 3863 rows of 2048 and 17 65 -> 53 us.  The order of every sum is the same.
+    constexpr int kBoth = ROWS > 1 ? 2 : 1;
+    for (int e0 = warp; e0 < experts + has_gate; e0 += kBoth * warps) {
+        const bool second = kBoth == 2 && e0 + warps < experts + has_gate;
+        const float* w[2] = {router + static_cast<size_t>(e0) * width, router + static_cast<size_t>(second ? e0 + warps : e0) * width};
+        float sums[kBoth][ROWS] = {};
         if (width % 4 == 0) {         // 16 bytes at a time (rows of the router and the shared rows start on 16-byte borders then)
-            const float4* w4 = reinterpret_cast<const float4*>(w);
             const float4* x4 = reinterpret_cast<const float4*>(xs);
 #pragma unroll ROWS == 1 ? 8 : 4
             for (int c = lane; c < width / 4; c += 32) {
-                const float4 a = w4[c];
+                float4 a[kBoth];
+#pragma unroll
+                for (int i = 0; i < kBoth; ++i) a[i] = reinterpret_cast<const float4*>(w[i])[c];
 #pragma unroll
                 for (int r = 0; r < ROWS; ++r) {
                     const float4 b = x4[r * (width / 4) + c];
-                    sums[r] = fmaf(a.x, b.x, sums[r]);
-                    sums[r] = fmaf(a.y, b.y, sums[r]);
-                    sums[r] = fmaf(a.z, b.z, sums[r]);
-                    sums[r] = fmaf(a.w, b.w, sums[r]);
+#pragma unroll
+                    for (int i = 0; i < kBoth; ++i) {
+                        sums[i][r] = fmaf(a[i].x, b.x, sums[i][r]);
+                        sums[i][r] = fmaf(a[i].y, b.y, sums[i][r]);
+                        sums[i][r] = fmaf(a[i].z, b.z, sums[i][r]);
+                        sums[i][r] = fmaf(a[i].w, b.w, sums[i][r]);
+                    }
                 }
             }
         } else {
             for (int c = lane; c < width; c += 32) {
 #pragma unroll
-                for (int r = 0; r < ROWS; ++r) sums[r] = fmaf(w[c], xs[static_cast<size_t>(r) * width + c], sums[r]);
+                for (int r = 0; r < ROWS; ++r)
+#pragma unroll
+                    for (int i = 0; i < kBoth; ++i) sums[i][r] = fmaf(w[i][c], xs[static_cast<size_t>(r) * width + c], sums[i][r]);
             }
         }
 #pragma unroll
-        for (int r = 0; r < ROWS; ++r) {
-            const float sum = mlr_warp_sum(sums[r]);
-            float* score = scores + static_cast<size_t>(r) * per_row;
-            float* choice = score + experts;
-            if (lane == 0 && row0 + r < rows) {
-                if (e >= experts) {
-                    shared_gate[row0 + r] = 1.0f / (1.0f + expf(-sum));
-                } else if (kind == 2) {
-                    score[e] = sum;
-                } else if (kind == 1) {
-                    score[e] = choice[e] = sum + (correction ? correction[e] : 0.0f);
-                } else {
-                    const float s = 1.0f / (1.0f + expf(-sum));
-                    score[e] = s;
-                    choice[e] = s + (correction ? correction[e] : 0.0f);
+        for (int i = 0; i < kBoth; ++i) {
+            const int e = e0 + i * warps;
+            if (i == 1 && !second) break;
+#pragma unroll
+            for (int r = 0; r < ROWS; ++r) {
+                const float sum = mlr_warp_sum(sums[i][r]);
+                float* score = scores + static_cast<size_t>(r) * per_row;
+                float* choice = score + experts;
+                if (lane == 0 && row0 + r < rows) {
+                    if (e >= experts) {
+                        shared_gate[row0 + r] = 1.0f / (1.0f + expf(-sum));
+                    } else if (kind == 2) {
+                        score[e] = sum;
+                    } else if (kind == 1) {
+                        score[e] = choice[e] = sum + (correction ? correction[e] : 0.0f);
+                    } else {
+                        const float s = 1.0f / (1.0f + expf(-sum));
+                        score[e] = s;
+                        choice[e] = s + (correction ? correction[e] : 0.0f);
+                    }
                 }
             }
         }

@@ -938,6 +938,7 @@ __global__ void __launch_bounds__(column_warps(DIM, RULE) * 32) recurrence_scan1
         }
     }
     mlr_grid_dependents_may_start();     // only now: blocks of the next grid that wait on this SM slow the walk
+    if (PASS == 2 && !last) return;      // the ends are the first pass's: blocks of later pieces, which may start after this one has ended, read them
     float* to = last ? my_state : end_of(first);
 #pragma unroll
     for (int n = 0; n < NC; ++n)

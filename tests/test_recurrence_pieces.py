@@ -7,12 +7,19 @@ import ctypes
 import pytest
 import torch
 
+from mini_llm_runtime_b200.ops.specs import RecurrenceSpec
+
 pytestmark = pytest.mark.gpu
 
 
 def _call(name, *args):
     from mini_llm_runtime_b200.ops import native
     native.call("recurrence", name, *args)
+
+
+def _stream():
+    from mini_llm_runtime_b200.ops import native
+    return native.stream()
 
 
 @pytest.mark.parametrize("rule,channel,dim,vdim,heads,segments", [
@@ -63,3 +70,32 @@ def test_pieces_give_what_the_whole_walk_gives(rule, channel, dim, vdim, heads, 
     assert torch.allclose(got_state, want_state, atol=1e-5 * scale, rtol=1e-5)
     assert torch.allclose(got, want, atol=2e-4, rtol=2e-4), float((got - want).abs().max())
     assert torch.equal(got_state[:, heads * vdim * dim:], start[:, heads * vdim * dim:])
+
+
+def test_the_second_pass_leaves_the_ends_alone():
+    """A block of a later piece puts the state before it together from the ends that the first pass left.  It may start after blocks of
+    earlier pieces have ended (their number is not bound by what the SMs hold at once), so those must not write ends of their own."""
+    g = torch.Generator().manual_seed(7)
+    heads, dim, vdim, rows, most, length = 2, 128, 32, 1000, 7, 144          # 7 pieces of 144 tokens, the last shorter
+    proj = torch.randn(rows, 2 * heads * dim + heads * vdim, generator=g).cuda()
+    decay = torch.tensor([0.99, 0.999], device="cuda")
+    spec = RecurrenceSpec(decay=decay.data_ptr(), heads=heads, qk_heads=heads, dim=dim, vdim=vdim, rule=RecurrenceSpec.RULE["decay"], norm_parts=heads,
+                          col_k=heads * dim, col_v=2 * heads * dim, q_mult=dim ** -0.5, k_mult=dim ** -0.5, unit_eps=1e-6, eps=1e-5, out_scale=1.0)
+    out, obuf = torch.empty(rows, heads * vdim, device="cuda"), torch.empty(rows, heads * vdim, device="cuda")
+    q, k = (torch.empty(rows, heads * dim, device="cuda") for _ in range(2))
+    ends = torch.full((rows // 128, heads, vdim + 1, dim), float("nan"), device="cuda")
+    state = torch.randn(1, heads * vdim * dim, generator=g).cuda()
+    positions = torch.arange(rows, dtype=torch.int32, device="cuda")
+    info = torch.tensor([[0, rows, 0, 0]], dtype=torch.int32, device="cuda")
+    common = (ctypes.addressof(spec), proj.data_ptr(), proj.stride(0), proj.data_ptr(), proj.stride(0), 0, out.data_ptr(), out.stride(0))
+    _call("mlr_linear_recurrence_pieces", *common, state.data_ptr(), state.stride(0), info.data_ptr(), 1, positions.data_ptr(), rows, q.data_ptr(),
+          k.data_ptr(), None, obuf.data_ptr(), None, None, 0, ends.data_ptr(), _stream())
+    for piece in range(1, most - 1):
+        alone = torch.zeros(1, heads * vdim * dim, device="cuda")            # the piece from a state of zero
+        info = torch.tensor([[piece * length, length, piece * length, 0]], dtype=torch.int32, device="cuda")
+        _call("mlr_linear_recurrence", *common, alone.data_ptr(), alone.stride(0), info.data_ptr(), 1, rows, None, None, _stream())
+        want = alone.view(heads, vdim, dim)
+        off = (ends[:, :, :vdim] - want).abs().amax((1, 2, 3))               # of every place of `ends`
+        place = int(off.nan_to_num(float("inf")).argmin())
+        assert float(off[place]) <= 1e-5 * float(want.abs().max())
+        assert torch.allclose(ends[place, :, vdim], (decay ** length)[:, None].expand(heads, dim), rtol=1e-4)

@@ -528,9 +528,33 @@ __global__ void __launch_bounds__(kFewThreads, 1) expert_few_kernel(const __nv_b
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     }
     mlr_grid_wait();
-    const int n = min(__ldcg(n_tiles), kFewMostTiles);
-    for (int i = threadIdx.x; i < 3 * n; i += kFewThreads) tile_of[i] = __ldcg(tiles + i);
-    __syncthreads();
+    int n = min(__ldcg(n_tiles), kFewMostTiles);
+    bool longer = false;
+    for (int i = threadIdx.x; i < 3 * n; i += kFewThreads) {
+        tile_of[i] = __ldcg(tiles + i);
+        longer = longer || (i % 3 == 2 && tile_of[i] > kFewRows);
+    }
+    if (__syncthreads_or(longer)) {
+        // A token whose scores are all NaN chose one expert `top` times: that expert's tile may have more than eight rows.  It is cut into
+        // tiles of eight, from the list's end on (a tile has at least one row, so the list's places last).
+        int cut = 0;
+        for (int i = 0; i < n; ++i) cut += (tile_of[3 * i + 2] + kFewRows - 1) / kFewRows;
+        cut = min(cut, kFewMostTiles);
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            int to = cut - 1;
+            for (int i = n - 1; i >= 0; --i) {
+                const int expert = tile_of[3 * i], row0 = tile_of[3 * i + 1], rows = tile_of[3 * i + 2];
+                for (int r = (rows - 1) / kFewRows * kFewRows; r >= 0 && to >= 0; r -= kFewRows, --to) {
+                    tile_of[3 * to] = expert;
+                    tile_of[3 * to + 1] = row0 + r;
+                    tile_of[3 * to + 2] = min(kFewRows, rows - r);
+                }
+            }
+        }
+        n = cut;
+        __syncthreads();
+    }
     constexpr int kOutputs = DUAL ? kFewUnit / 2 : kFewUnit;              // of a unit
     const int per_tile = (N + kOutputs - 1) / kOutputs, units = n * per_tile;
     const int first = static_cast<int>(static_cast<long long>(units) * blockIdx.x / gridDim.x);
@@ -573,7 +597,7 @@ __global__ void __launch_bounds__(kFewThreads, 1) expert_few_kernel(const __nv_b
     int tile = -1, row0 = 0, rows = 0, parity = 0, i = 0;
     for (int unit = first; unit < last; ++unit) {
         if (unit / per_tile != tile) {
-            tile = unit / per_tile, row0 = tile_of[3 * tile + 1], rows = min(tile_of[3 * tile + 2], kFewRows);
+            tile = unit / per_tile, row0 = tile_of[3 * tile + 1], rows = tile_of[3 * tile + 2];
             const int r = row0 + min(g, rows - 1);
             const __nv_bfloat16* row = a + static_cast<long long>(source ? __ldcg(source + r) / divisor : r) * lda;
 #pragma unroll

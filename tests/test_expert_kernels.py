@@ -13,6 +13,11 @@ def _call(module, name, *args):
     native.call(module, name, *args)
 
 
+def _stream():
+    from mini_llm_runtime_b200.ops import native
+    return native.stream()
+
+
 def _listed(choices, experts, tile_rows):
     """choices [rows, top] (an expert past the last: none).  Tiles, their number, the pairs in the order by expert."""
     tiles, order = [], []
@@ -62,6 +67,40 @@ def test_few_rows(rows, experts, top, N, K, kind):
         assert torch.allclose(plain[first:first + count].double(), y, atol=1e-4, rtol=1e-4)
         assert torch.allclose(act[first:first + count].double(), _gate(y, up, kind, *shape), atol=1e-3, rtol=4e-3)
     assert torch.isnan(plain[len(order):]).all() and torch.isnan(act[len(order):].float()).all() and status.item() == 0
+
+
+@pytest.mark.parametrize("experts,top,lost", [(16, 4, [3]), (16, 16, [0]), (9, 5, [0, 2, 4, 6, 7]), (40, 32, [1, 2, 5])])
+def test_few_rows_beside_one_without_scores(experts, top, lost):
+    """A token that is all NaN has no best expert and takes the first one `top` times, which then has more rows than the step.  The other
+    tokens get the bits that they get beside ordinary tokens, and its own rows are NaN and not what the buffers held before."""
+    rows, N, K = 8, 72, 520
+    g = torch.Generator().manual_seed(experts + top)
+    draw = lambda *shape, scale=1.0: (torch.randn(*shape, generator=g) * scale).bfloat16().cuda()
+    plain, w, w2, down = draw(rows, K), draw(experts, N, K, scale=K ** -0.5), draw(experts, N, K, scale=K ** -0.5), draw(experts, K, N, scale=N ** -0.5)
+    router, counts = torch.randn(experts, K, generator=g).cuda(), torch.zeros(experts, dtype=torch.int32, device="cuda")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    broken = plain.clone()
+    broken[lost] = float("nan")
+    results = []
+    for x in (plain, broken):
+        on = lambda n, dtype=torch.int32: torch.full((n,), -1, dtype=dtype, device="cuda")
+        chosen, place, row_of_pair, pair_of_row = (on(rows * top) for _ in range(4))
+        weights, first_row, tiles, n_tiles = on(rows * top, torch.float32), on(experts + 1), on(3 * (rows * top // 32 + experts)), on(1)
+        _call("experts", "mlr_experts_route", x.data_ptr(), K, 1, router.data_ptr(), None, rows, K, experts, experts, 1, 1, top, 0, chosen.data_ptr(),
+              weights.data_ptr(), place.data_ptr(), counts.data_ptr(), None, None, 0, _stream())
+        _call("experts", "mlr_experts_arrange", counts.data_ptr(), chosen.data_ptr(), place.data_ptr(), experts, rows, top, 32, first_row.data_ptr(),
+              tiles.data_ptr(), n_tiles.data_ptr(), row_of_pair.data_ptr(), pair_of_row.data_ptr(), _stream())
+        act, y = torch.full((rows * top, N), 7.0, dtype=torch.bfloat16, device="cuda"), torch.full((rows * top, K), 7.0, device="cuda")
+        _call("experts", "mlr_experts_product_few", x.data_ptr(), K, pair_of_row.data_ptr(), top, w.data_ptr(), w2.data_ptr(), 1, N, K, act.data_ptr(), N,
+              tiles.data_ptr(), n_tiles.data_ptr(), rows, top, 0.0, 0.0, 0.0, status.data_ptr(), _stream())
+        _call("experts", "mlr_experts_product_few", act.data_ptr(), N, None, 1, down.data_ptr(), None, 0, K, N, y.data_ptr(), K, tiles.data_ptr(),
+              n_tiles.data_ptr(), rows, top, 0.0, 0.0, 0.0, status.data_ptr(), _stream())
+        results.append(y[row_of_pair.long()].view(rows, top, K))
+        most = int(tiles.view(-1, 3)[:n_tiles.item(), 2].max())
+    sound = [r for r in range(rows) if r not in lost]
+    assert most > (8 if len(lost) * top > 8 else 1) and status.item() == 0
+    assert torch.equal(results[1][sound], results[0][sound])
+    assert torch.isnan(results[1][lost]).all()
 
 
 @pytest.mark.parametrize("rows,experts,top,N,K,kind", [(1, 1, 1, 128, 64, 1), (300, 1, 1, 256, 128, 2), (257, 3, 2, 136, 72, 1), (700, 16, 4, 264, 520, 2),

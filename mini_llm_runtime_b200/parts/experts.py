@@ -139,7 +139,7 @@ class RoutedExperts(FeedForward):
             if grouped:
                 b.launch("gemm_bf16_tcgen05_pair", "mlr_grouped_product_bf16", side.ptr if source is not None else a, K, rows, top, w, w2, E, kind, N, K, out, N,
                          tiles.ptr, n_tiles.ptr, *shape, b.status, b.stream)
-            elif few and lib.mlr_experts_few(K, lda):
+            elif few and a % 16 == 0 and lib.mlr_experts_few(K, lda):
                 b.launch("experts", "mlr_experts_product_few", a, lda, source, divisor, w, w2, kind, N, K, out, N, tiles.ptr, n_tiles.ptr, rows, top,
                          *shape, b.status, b.stream)
             else:

@@ -137,3 +137,30 @@ def test_many_rows_on_two_sms(rows, experts, top, N, K, kind):
         assert torch.allclose(act[first:first + n].double(), want, atol=1e-3, rtol=4e-3)
         assert torch.allclose(y[first:first + n].double(), act[first:first + n].double() @ down[e].double().T, atol=1e-4, rtol=1e-4)
     assert torch.isnan(act[count:].float()).all() and torch.isnan(y[count:]).all() and status.item() == 0
+
+
+@pytest.mark.parametrize("offset", [1, 3])
+def test_the_part_takes_rows_off_16_byte_borders(offset):
+    """A caller's activations may be a view that starts anywhere: the first product then leaves the kernel that copies 16 bytes at a time.
+    Sums in another order ahead of two roundings to bfloat16 (2^-9 each): a hundredth of the results' size."""
+    from mini_llm_runtime_b200.config.base import PartSpec
+    from mini_llm_runtime_b200.csrc import build
+    from mini_llm_runtime_b200.engine.runtime import Runtime
+    from mini_llm_runtime_b200.parts.base import StepContext
+    from mini_llm_runtime_b200.parts.experts import RoutedExperts
+    rows, width, inter, experts, top = 4, 64, 48, 6, 2
+    g = torch.Generator().manual_seed(offset)
+    names, tensors = {"router": "r", "correction": "c"}, {"r": torch.randn(experts, width, generator=g), "c": torch.zeros(experts)}
+    for e in range(experts):
+        for role, shape in (("gate", (inter, width)), ("up", (inter, width)), ("down", (width, inter))):
+            names[f"e{e}.{role}"] = f"e{e}.{role}"
+            tensors[f"e{e}.{role}"] = torch.randn(*shape, generator=g) * shape[1] ** -0.5
+    rt = Runtime(torch.bfloat16)
+    part = RoutedExperts(PartSpec("routed_experts", {"hidden_size": width, "intermediate_size": inter, "experts": experts, "top": top}, names))
+    build.ensure(part.kernel_modules(rt.dtype) + ["host"])
+    part.bind({k: v.bfloat16() for k, v in tensors.items()}, rt)
+    step = StepContext(rt=rt, num_rows=rows, segments=[], token_ids=None, positions=None, segment_of_row=None, segment_info=None, slots=None, tables={},
+                       page_size=16, status=torch.zeros(1, dtype=torch.int32, device="cuda"))
+    x = torch.randn(rows, width + 8, generator=g).bfloat16().cuda()[:, offset:offset + width]
+    got, want = part.forward(x, step), part.forward(x.contiguous(), step)
+    assert torch.allclose(got, want, atol=1e-2 * float(want.abs().max()), rtol=0)

@@ -117,13 +117,14 @@ __global__ void __launch_bounds__(T::kThreads) gemm_f32_tile_kernel(const float*
 }
 
 // ---- up to four rows (a decode step): a pass over W.  A block takes BN rows of W; thread (n, g) has row n of them and the rows g, g + G,
-// .. of A, G = 128 / BN.  W's first stages are on their way before the kernel before this one has ended (no kernel writes weights).
+// .. of A, G = 128 / BN.  With `static_w` (no kernel in flight writes W: it holds weights) W's first stages are on their way before the
+// kernel before this one has ended.
 constexpr int kFewRows = 4, kFewThreads = 128, kFewK = 64, kFewLd = kFewK + 4;
 constexpr size_t few_shared(int bn, int stages, int rows) { return sizeof(float) * stages * (bn + rows) * kFewLd; }
 
 template <bool kVector, int BN, int STAGES, int MT>
 __global__ void __launch_bounds__(kFewThreads) gemm_f32_few_kernel(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw,
-                                                                   int ldc) {
+                                                                   int ldc, int static_w) {
     extern __shared__ __align__(16) float staged[];           // per stage: W [BN][kFewLd], A [M][kFewLd]
     constexpr int kGroups = kFewThreads / BN, kChunks = kFewK / 4;
     const int tid = threadIdx.x, n = tid % BN, g = tid / BN;
@@ -144,8 +145,9 @@ __global__ void __launch_bounds__(kFewThreads) gemm_f32_few_kernel(const float* 
             stage4<kVector>(to + r * kFewLd + c, A + static_cast<size_t>(r) * lda, step * kFewK + c, K, true);
         }
     };
+    if (!static_w) mlr_grid_wait();
     for (int step = 0; step < STAGES - 1 && step < steps; ++step) fetch_w(step);
-    mlr_grid_wait();
+    if (static_w) mlr_grid_wait();
     // The first group to complete holds all of W's first stages and A's first; the later ones A's alone.
     for (int step = 0; step < STAGES - 1; ++step) {
         if (step < steps) fetch_a(step);
@@ -190,7 +192,7 @@ int allow_shared(Kernel kernel, size_t bytes) {
 struct Product {
     const float *A, *W;
     float* C;
-    int M, N, K, lda, ldw, ldc;
+    int M, N, K, lda, ldw, ldc, static_w;
     cudaStream_t stream;
 };
 
@@ -207,7 +209,7 @@ template <bool kVector, int BN, int STAGES, int MT>
 int launch_few(const Product& p) {
     if (allow_shared(gemm_f32_few_kernel<kVector, BN, STAGES, MT>, few_shared(BN, STAGES, kFewRows))) return 1;
     mlr_launch((gemm_f32_few_kernel<kVector, BN, STAGES, MT>), dim3((p.N + BN - 1) / BN), dim3(kFewThreads), few_shared(BN, STAGES, p.M), p.stream, p.A, p.W,
-               p.C, p.M, p.N, p.K, p.lda, p.ldw, p.ldc);
+               p.C, p.M, p.N, p.K, p.lda, p.ldw, p.ldc, p.static_w);
     return 0;
 }
 
@@ -246,16 +248,26 @@ int choose(const Product& p) {
                            Tile<16, 64, 2, 4, 4, 64>, Tile<16, 128, 8, 4, 4>, Tile<8, 128, 4, 4, 4>, Tile<16, 32, 2, 2, 5, 64>, Tile<8, 32, 1, 2, 5, 64>>(p);
 }
 
-}  // namespace
-
-MLR_API int mlr_gemm_f32(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw,
-                         int ldc, cudaStream_t stream) {
+int product(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw, int ldc, int static_w, cudaStream_t stream) {
     MLR_REQUIRE(M >= 0 && N > 0 && K > 0, "gemm_f32: bad sizes M=%d N=%d K=%d", M, N, K);
     MLR_REQUIRE(lda >= K && ldw >= K && ldc >= N, "gemm_f32: a leading dimension is smaller than its row");
     if (M == 0) return 0;
     const bool vector = lda % 4 == 0 && ldw % 4 == 0 && reinterpret_cast<uintptr_t>(A) % 16 == 0 &&
                         reinterpret_cast<uintptr_t>(W) % 16 == 0;
-    const Product p = {A, W, C, M, N, K, lda, ldw, ldc, stream};
+    const Product p = {A, W, C, M, N, K, lda, ldw, ldc, static_w, stream};
     if (vector ? choose<true>(p) : choose<false>(p)) return 1;
     return mlr_launched("gemm_f32");
+}
+
+}  // namespace
+
+MLR_API int mlr_gemm_f32(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw,
+                         int ldc, cudaStream_t stream) {
+    return product(A, W, C, M, N, K, lda, ldw, ldc, 0, stream);
+}
+
+// The same for a W that no kernel in flight writes (it holds weights): a few-row product fetches it before the kernels before it are done.
+MLR_API int mlr_gemm_f32_weights(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw,
+                                 int ldc, cudaStream_t stream) {
+    return product(A, W, C, M, N, K, lda, ldw, ldc, 1, stream);
 }

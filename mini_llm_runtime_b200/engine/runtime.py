@@ -349,7 +349,7 @@ class Runtime:
             return out
         x = self.materialize(b, x)
         if self.dtype is torch.float32:
-            b.launch("gemm_f32", "mlr_gemm_f32", x.ptr, w.data_ptr(), out.ptr, x.rows, N, K, x.ld, w.stride(0), out.ld, b.stream,
+            b.launch("gemm_f32", "mlr_gemm_f32_weights", x.ptr, w.data_ptr(), out.ptr, x.rows, N, K, x.ld, w.stride(0), out.ld, b.stream,
                      need=b.need_for(x.rows))
         elif self._pair(b, x, w):
             self._pair_launch(b, x, w, out, "bf16" if out.dtype is torch.bfloat16 else "f32")

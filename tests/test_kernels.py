@@ -180,6 +180,22 @@ def test_gemm_f32_every_tile_gives_the_bits_of_a_row_alone(M, N, K, aligned):
         assert torch.equal(alone[0], out[row]), row
 
 
+@pytest.mark.parametrize("M,N,K", [(1, 3000, 512), (2, 20000, 256), (4, 20000, 200), (3, 500, 1024)])
+def test_gemm_f32_takes_a_result_as_its_second_operand(M, N, K):
+    """Two products back to back, the second over the first's result where weights would stand: it waits for it like for its rows."""
+    a, w = torch.randn(N, 64, generator=gen(4)).to(DEV), torch.randn(K, 64, generator=gen(5)).to(DEV)
+    x = torch.randn(M, K, generator=gen(6)).to(DEV)
+    made, out, want = torch.empty(N, K, device=DEV), torch.empty(M, N, device=DEV), torch.empty(M, N, device=DEV)
+    F().gemm_f32(a, w, made)
+    torch.cuda.synchronize()
+    F().gemm_f32(x, made, want)
+    for _ in range(5):
+        made.fill_(float("nan"))
+        F().gemm_f32(a, w, made)
+        F().gemm_f32(x, made, out)
+        assert torch.equal(out, want)
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 64, 64), (8, 4096, 4096), (3, 100, 96), (16, 515, 1056), (64, 300, 200), (65, 256, 64),
                                    (128, 256, 4096), (200, 515, 136), (2048, 6144, 4096), (300, 48, 12288), (129, 24, 72)])
 @pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])

@@ -18,6 +18,8 @@
 // each from different banks.
 #include "common.cuh"
 
+#include <climits>
+
 namespace {
 
 // 16 bytes at column k of a row of K values, zeros past its end.
@@ -56,8 +58,8 @@ __global__ void __launch_bounds__(T::kThreads) gemm_f32_tile_kernel(const float*
     extern __shared__ __align__(16) float staged[];           // per stage: A [BM][kLd], W [BN][kLd]
     constexpr int kAcross = BN / TN, kDown = BM / TM, kStage = (BM + BN) * T::kLd, kChunks = T::kK / 4;
     const int tid = threadIdx.x, tx = tid % kAcross, ty = tid / kAcross;
-    // Neighbouring blocks share W's rows, so that they come from memory once.
-    const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
+    // Neighbouring blocks share W's rows, so that they come from memory once.  All tiles in one dimension of the grid: the others take 65535.
+    const int row_tiles = (M + BM - 1) / BM, m0 = blockIdx.x % row_tiles * BM, n0 = blockIdx.x / row_tiles * BN;
     const int steps = (K + T::kK - 1) / T::kK;
     auto fetch_a = [&](int step) {
         float* to = staged + (step % T::kStages) * kStage;
@@ -198,10 +200,10 @@ struct Product {
 
 template <bool kVector, typename T>
 int launch_tile(const Product& p) {
-    const dim3 grid((p.M + T::kRows - 1) / T::kRows, (p.N + T::kColumns - 1) / T::kColumns);
-    MLR_REQUIRE(grid.y <= 65535, "gemm_f32: N=%d needs more than 65535 column tiles", p.N);
+    const long long blocks = ((p.M + T::kRows - 1LL) / T::kRows) * ((p.N + T::kColumns - 1LL) / T::kColumns);
+    MLR_REQUIRE(blocks <= INT_MAX, "gemm_f32: M=%d N=%d need more than %d tiles", p.M, p.N, INT_MAX);
     if (allow_shared(gemm_f32_tile_kernel<kVector, T>, T::kShared)) return 1;
-    mlr_launch((gemm_f32_tile_kernel<kVector, T>), grid, dim3(T::kThreads), T::kShared, p.stream, p.A, p.W, p.C, p.M, p.N, p.K, p.lda, p.ldw, p.ldc);
+    mlr_launch((gemm_f32_tile_kernel<kVector, T>), dim3(static_cast<unsigned>(blocks)), dim3(T::kThreads), T::kShared, p.stream, p.A, p.W, p.C, p.M, p.N, p.K, p.lda, p.ldw, p.ldc);
     return 0;
 }
 

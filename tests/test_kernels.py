@@ -180,6 +180,14 @@ def test_gemm_f32_every_tile_gives_the_bits_of_a_row_alone(M, N, K, aligned):
         assert torch.equal(alone[0], out[row]), row
 
 
+@pytest.mark.parametrize("M,N,K", [(5, 65535 * 32 + 1, 4), (65535 * 64, 3, 4), (1, 65535 * 64 + 1, 4)])
+def test_gemm_f32_takes_more_tiles_than_a_grid_has_rows(M, N, K):
+    a, w = torch.randint(-8, 9, (M, K), generator=gen(7)).float().to(DEV), torch.randint(-8, 9, (N, K), generator=gen(8)).float().to(DEV)
+    out = torch.full((M, N), float("nan"), device=DEV)
+    F().gemm_f32(a, w, out)
+    assert torch.equal(out, (a.double() @ w.double().T).float())           # small whole numbers: exact
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 3000, 512), (2, 20000, 256), (4, 20000, 200), (3, 500, 1024)])
 def test_gemm_f32_takes_a_result_as_its_second_operand(M, N, K):
     """Two products back to back, the second over the first's result where weights would stand: it waits for it like for its rows."""

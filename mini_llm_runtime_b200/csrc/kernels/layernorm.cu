@@ -8,13 +8,14 @@
 // `history` holds the stream's earlier states of this step, [states][rows][width] float32, `slot_stride` values apart: state 0
 // is what the embedding made, state j + 1 what layer j computed before its own averaging.  A launch with n_prev = 0 and w = {1}
 // starts the history (it stores the stream as state 0).  Everything is float32; `out` is float32 or bfloat16.  One block per
-// row, the row in shared memory, sums by a fixed tree (a row's result depends on that row only).
+// row, the row in registers or in shared memory, sums by a fixed tree (a row's result depends on that row only).
 #include "common.cuh"
 
 namespace {
 
 constexpr int kThreads = 256;
 
+// The row in shared memory: rows too wide for the kernel below, and results or norm weights that start off the borders it wants.
 template <typename TO>
 __global__ void __launch_bounds__(kThreads) depth_norm_kernel(float* h, const float* d1, long long ld1, const float* d2, long long ld2,
                                                               const float* bias, float* history, long long slot_stride, int n_prev,
@@ -27,6 +28,7 @@ __global__ void __launch_bounds__(kThreads) depth_norm_kernel(float* h, const fl
     const int r = blockIdx.x;
     const int row = want_rows ? want_rows[r] : r;
     float* hrow = h + static_cast<size_t>(row) * width;
+    const bool vec = width % 4 == 0 && ld1 % 4 == 0 && ld2 % 4 == 0 && slot_stride % 4 == 0;
     float sum = 0.0f;
     auto value_at = [&](int c, float x) {
         // x: the stream's value; returns what the stream becomes
@@ -45,11 +47,68 @@ __global__ void __launch_bounds__(kThreads) depth_norm_kernel(float* h, const fl
         }
         return x;
     };
-    for (int c = threadIdx.x; c < width; c += kThreads) {
-        const float v = value_at(c, __ldcg(hrow + c));
-        if (store_h) hrow[c] = v;
-        xs[c] = v;
-        sum += v;
+    if (vec) {
+        for (int c = threadIdx.x * 4; c < width; c += kThreads * 4) {
+            float4 x = __ldcg(reinterpret_cast<const float4*>(hrow + c));
+            float v[4] = {x.x, x.y, x.z, x.w};
+            float add[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            bool any = false;
+            if (d1) {
+                const float4 a = __ldcg(reinterpret_cast<const float4*>(d1 + static_cast<size_t>(row) * ld1 + c));
+                add[0] = a.x; add[1] = a.y; add[2] = a.z; add[3] = a.w;
+                any = true;
+            }
+            if (d2) {
+                const float4 a = __ldcg(reinterpret_cast<const float4*>(d2 + static_cast<size_t>(row) * ld2 + c));
+                add[0] += a.x; add[1] += a.y; add[2] += a.z; add[3] += a.w;
+                any = true;
+            }
+            if (bias) {
+                const float4 a = *reinterpret_cast<const float4*>(bias + c);
+                add[0] += a.x; add[1] += a.y; add[2] += a.z; add[3] += a.w;
+                any = true;
+            }
+            if (any) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) v[e] += add[e];
+            }
+            if (history) {
+                float* slot = history + static_cast<size_t>(row) * width + c;
+                *reinterpret_cast<float4*>(slot + static_cast<size_t>(n_prev) * slot_stride) = make_float4(v[0], v[1], v[2], v[3]);
+                float mixed[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                int j = 0;
+                for (; j + 4 <= n_prev; j += 4) {      // four states on their way at a time
+                    float4 s[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) s[u] = __ldcg(reinterpret_cast<const float4*>(slot + static_cast<size_t>(j + u) * slot_stride));
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        const float w = dwa[j + u];
+                        mixed[0] = fmaf(w, s[u].x, mixed[0]); mixed[1] = fmaf(w, s[u].y, mixed[1]);
+                        mixed[2] = fmaf(w, s[u].z, mixed[2]); mixed[3] = fmaf(w, s[u].w, mixed[3]);
+                    }
+                }
+                for (; j < n_prev; ++j) {
+                    const float4 s = __ldcg(reinterpret_cast<const float4*>(slot + static_cast<size_t>(j) * slot_stride));
+                    const float w = dwa[j];
+                    mixed[0] = fmaf(w, s.x, mixed[0]); mixed[1] = fmaf(w, s.y, mixed[1]);
+                    mixed[2] = fmaf(w, s.z, mixed[2]); mixed[3] = fmaf(w, s.w, mixed[3]);
+                }
+                const float w = dwa[n_prev];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) v[e] = fmaf(w, v[e], mixed[e]);
+            }
+            if (store_h) *reinterpret_cast<float4*>(hrow + c) = make_float4(v[0], v[1], v[2], v[3]);
+            *reinterpret_cast<float4*>(xs + c) = make_float4(v[0], v[1], v[2], v[3]);
+            sum += (v[0] + v[1]) + (v[2] + v[3]);
+        }
+    } else {
+        for (int c = threadIdx.x; c < width; c += kThreads) {
+            const float v = value_at(c, __ldcg(hrow + c));
+            if (store_h) hrow[c] = v;
+            xs[c] = v;
+            sum += v;
+        }
     }
     if (!out) return;
     const float mean = mlr_block_sum(sum, scratch) / static_cast<float>(width);

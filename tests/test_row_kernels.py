@@ -70,6 +70,28 @@ def test_depth_average_and_layer_norm(dtype, width, states):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("width,states,off,gap", [(16388, 1, 0, 0), (20480, 6, 0, 0), (2048, 3, 1, 0), (4100, 5, 2, 0), (1030, 2, 0, 0), (1024, 4, 0, 2)])
+def test_depth_average_and_layer_norm_of_other_rows(dtype, width, states, off, gap):
+    """Rows wider than a thread's registers take, results and norm weights `off` a border, results to add whose rows lie `gap` off one."""
+    from mini_llm_runtime_b200.ops import native
+    draw, rows = _draw(width + states), 3
+    history, h, d1, w = draw(states + 2, rows, width), draw(rows, width), draw(rows, width + gap)[:, :width], draw(width + off)[off:]
+    b, dwa = draw(width + off)[off:], draw(states + 1)
+    old, before = h.double(), history.clone()
+    out = torch.empty(rows, width + off, dtype=dtype, device="cuda")[:, off:]
+    _call("layernorm", "mlr_depth_norm", h.data_ptr(), d1.data_ptr(), d1.stride(0), None, 0, None, history.data_ptr(), history.stride(0), states,
+          dwa.data_ptr(), w.data_ptr(), b.data_ptr(), 1e-5, out.data_ptr(), out.stride(0), native.is_bf16(out), None, rows, width, 1, native.stream())
+    newest = old + d1.double()
+    stream = (torch.cat([before[:states].double(), newest[None]]) * dwa.double()[:, None, None]).sum(0)
+    centred = stream - stream.mean(-1, keepdim=True)
+    want = centred / (centred.square().mean(-1, keepdim=True) + 1e-5).sqrt() * w.double() + b.double()
+    _near(history[states], newest, torch.float32)
+    assert torch.equal(history[:states], before[:states]) and torch.equal(history[states + 1:], before[states + 1:])
+    _near(h, stream, torch.float32)
+    _near(out, want, dtype)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("width,groups", [(128, 1), (1024, 8), (1152, 3), (2048, 1), (2048, 4), (4096, 32), (5120, 4), (8192, 1)])
 def test_grouped_norms_around_a_sub_layer(dtype, width, groups):
     """The result normed and added into the stream, the sum normed, and a result in pieces."""

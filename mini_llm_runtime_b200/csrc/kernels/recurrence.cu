@@ -681,9 +681,9 @@ __host__ __device__ constexpr int column_warps(int dim, int rule) { return kScan
 // of zero, without outputs, and leaves their ends and the products of their decays in `ends`; pass 2 puts the state before each later
 // piece together from those and walks the piece.  The walk of one request's 2048 tokens over 8 heads has 64 blocks for 148 SMs and every
 // token waits for the one before: 2048 rows 270 us whole, 60 + 90 us in 16 pieces.
-constexpr int kLeastPiece = 128;          // tokens of a piece at least: `ends` has a place for every 128 rows
+constexpr int kLeastPiece = 128;          // tokens of a piece at least
 struct WalkPieces {
-    float* ends;                          // [rows / 128][heads][(vdim + 1)][dim]: a piece's end by column, then its decays' products
+    float* ends;                          // [segments * most][heads][(vdim + 1)][dim]: a piece's end by column, then its decays' products
     int most;                             // pieces of a segment
 };
 __host__ __device__ inline size_t ends_of_piece(const RecurrenceSpec& s) { return static_cast<size_t>(s.heads) * (s.vdim + 1) * s.dim; }
@@ -710,7 +710,6 @@ __global__ void __launch_bounds__(column_warps(DIM, RULE) * 32) recurrence_scan1
     const int slot = segment_info[4 * segment + 3];
     int piece = 0, piece_rows = count;
     bool last = true;                     // of the segment's pieces: its end is the segment's
-    const int segment_first = first;
     if (PASS) {
         piece = blockIdx.x % pieces.most;
         piece_rows = max(kLeastPiece, ((count + pieces.most - 1) / pieces.most + 3) / 4 * 4);
@@ -743,16 +742,13 @@ __global__ void __launch_bounds__(column_warps(DIM, RULE) * 32) recurrence_scan1
 #pragma unroll
         for (int j = 0; j < H; ++j) S[n][j] = live(n) && piece == 0 ? pair_at(my_state + n * kScanBlockCols * DIM + place(2 * j)) : twice(0.0f);
     // The end of a piece for this lane's columns, and the products of its decays.
-    auto end_of = [&](int piece_first) {
-        return pieces.ends + piece_first / kLeastPiece * ends_of_piece(s) + (static_cast<size_t>(head) * (s.vdim + 1) + block_col + my_col) * DIM;
-    };
-    auto decays_of = [&](int piece_first) {
-        return pieces.ends + piece_first / kLeastPiece * ends_of_piece(s) + (static_cast<size_t>(head) * (s.vdim + 1) + s.vdim) * DIM;
-    };
+    auto place_of = [&](int p) { return pieces.ends + (static_cast<size_t>(segment) * pieces.most + p) * ends_of_piece(s); };
+    auto end_of = [&](int p) { return place_of(p) + (static_cast<size_t>(head) * (s.vdim + 1) + block_col + my_col) * DIM; };
+    auto decays_of = [&](int p) { return place_of(p) + (static_cast<size_t>(head) * (s.vdim + 1) + s.vdim) * DIM; };
     if (PASS == 2) {
         for (int before = 0; before < piece; ++before) {
-            const float* end = end_of(segment_first + before * piece_rows);
-            const float* d = decays_of(segment_first + before * piece_rows);
+            const float* end = end_of(before);
+            const float* d = decays_of(before);
 #pragma unroll
             for (int j = 0; j < H; ++j) {
                 const float2 decayed = before > 0 ? __ldcg(reinterpret_cast<const float2*>(d + place(2 * j))) : twice(0.0f);      // nothing lies before the first piece
@@ -939,7 +935,7 @@ __global__ void __launch_bounds__(column_warps(DIM, RULE) * 32) recurrence_scan1
     }
     mlr_grid_dependents_may_start();     // only now: blocks of the next grid that wait on this SM slow the walk
     if (PASS == 2 && !last) return;      // the ends are the first pass's: blocks of later pieces, which may start after this one has ended, read them
-    float* to = last ? my_state : end_of(first);
+    float* to = last ? my_state : end_of(piece);
 #pragma unroll
     for (int n = 0; n < NC; ++n)
         if (live(n)) {
@@ -952,7 +948,7 @@ __global__ void __launch_bounds__(column_warps(DIM, RULE) * 32) recurrence_scan1
         }
     if (track && !last && lane < kColumnLanes) {
 #pragma unroll
-        for (int j = 0; j < H; ++j) *reinterpret_cast<float2*>(decays_of(first) + place(2 * j)) = product[PASS == 1 ? j : 0];
+        for (int j = 0; j < H; ++j) *reinterpret_cast<float2*>(decays_of(piece) + place(2 * j)) = product[PASS == 1 ? j : 0];
     }
 }
 
@@ -1190,11 +1186,48 @@ MLR_API int mlr_linear_recurrence(const RecurrenceSpec* spec, const void* proj, 
     return mlr_launched("linear_recurrence");
 }
 
+namespace {
+
+// How the walk of a step is launched: column blocks per head, and the pieces of a segment.
+struct WalkShape {
+    bool fixed_size, two;                 // `two`: two state columns a lane
+    int block_cols, column_blocks, pieces;
+};
+
+WalkShape walk_shape(const RecurrenceSpec& s, int n_segments, int rows) {
+    WalkShape w = {};
+    w.fixed_size = s.dim == 32 || s.dim == 64 || s.dim == 96 || s.dim == 128 || s.dim == 256;
+    const int columns = (s.vdim + kScanBlockCols - 1) / kScanBlockCols;
+    // The step rule's walk takes two state columns a lane where blocks of sixteen columns would outnumber the SMs.
+    w.two = s.rule == 2 && w.fixed_size && columns > 1 && static_cast<long long>(n_segments) * s.heads * columns > mlr_sm_count();
+    w.block_cols = kScanBlockCols * (w.two ? 2 : 1);
+    w.column_blocks = (s.vdim + w.block_cols - 1) / w.block_cols;
+    // Pieces where whole segments leave the SMs short of blocks: up to eight blocks an SM, and at least six pieces (the two passes take
+    // the time of two pieces, and pieces slow one another).  Measured at 2048 rows of 128 x 128: 64 blocks in 16 pieces 270 -> 150 us,
+    // 128 blocks (two requests) in 9 pieces 281 -> 235 us; 256 blocks in 4 pieces 433 -> 580 us.
+    const long long blocks = static_cast<long long>(n_segments) * s.heads * w.column_blocks;
+    const long long most = std::min(std::min(8ll * mlr_sm_count() / blocks, static_cast<long long>(rows / n_segments / kLeastPiece)), 16ll);
+    w.pieces = s.rule != 1 && w.fixed_size && most >= 6 ? static_cast<int>(most) : 1;
+    return w;
+}
+
+}  // namespace
+
+// The most ends of pieces a step of up to `rows` rows leaves (0: none is walked in pieces): places of heads * (vdim + 1) * dim values.
+MLR_API int mlr_linear_recurrence_places(const RecurrenceSpec* spec, int rows) {
+    int most = 0;
+    for (int n = 1; n <= rows / (6 * kLeastPiece) && n <= 8 * mlr_sm_count() / 6; ++n) {
+        const int pieces = walk_shape(*spec, n, rows).pieces;
+        if (pieces > 1) most = std::max(most, n * pieces);
+    }
+    return most;
+}
+
 // The three-kernel form.  qf, kf: float32 [rows, qk_heads * dim]; gates: float32 [rows, 2 * heads] (delta and step rules; else unused);
 // obuf: float32 [rows, heads * vdim].  Same results as `mlr_linear_recurrence` up to the order in which a column's sums are added
 // (the same order for head sizes that are no multiple of 32).  With a decay per channel, df [rows, heads * dim] and (low-rank gate) gf
 // [rows, heads * vdim] are float32 room; with `products_made` they hold the low-rank products' results already (df without the bias).
-// ends: float32 room for the ends of a walk's pieces, rows / 128 times heads * (vdim + 1) * dim values, or null (segments are walked whole).
+// ends: float32 room for the ends of a walk's pieces (`mlr_linear_recurrence_places`), or null (segments are walked whole).
 MLR_API int mlr_linear_recurrence_pieces(const RecurrenceSpec* spec, const void* proj, int ld, const void* side, int ld_side, int act_bf16,
                                          void* out, int ld_out, float* state, long long state_stride, const int* segment_info,
                                          int n_segments, const int* positions, int rows, float* qf, float* kf, float* gates, float* obuf,
@@ -1208,32 +1241,22 @@ MLR_API int mlr_linear_recurrence_pieces(const RecurrenceSpec* spec, const void*
     if (n_segments == 0 || rows == 0) return 0;
     const int regs = s.dim <= 32 ? 1 : s.dim <= 64 ? 2 : s.dim <= 128 ? 4 : 8;
     const bool channel = s.channel_decay != 0;
+    const WalkShape shape = walk_shape(s, n_segments, rows);
+    const bool fixed_size = shape.fixed_size, two = shape.two;
+    const int block_cols = shape.block_cols;
     // q and k (and the channels' decays) in two stages
-    // The step rule's walk takes two state columns a lane where blocks of sixteen columns would outnumber the SMs.
-    const bool fixed_size = s.dim == 32 || s.dim == 64 || s.dim == 96 || s.dim == 128 || s.dim == 256;
-    const int column_blocks = (s.vdim + kScanBlockCols - 1) / kScanBlockCols;
-    const bool two = s.rule == 2 && fixed_size && column_blocks > 1 && static_cast<long long>(n_segments) * s.heads * column_blocks > mlr_sm_count();
-    const int block_cols = kScanBlockCols * (two ? 2 : 1);
     const size_t per_token = sizeof(float) * ((channel ? 6 : 4) * static_cast<size_t>(s.dim) + 2 * block_cols + 2);
     int batch = static_cast<int>(((channel ? 84 : 72) * 1024) / per_token);
     batch = batch < 1 ? 1 : (batch > 32 ? 32 : batch);
     if (batch > 4) batch -= batch % 4;
     const size_t shared = per_token * batch + (channel ? 16 : 0);
-    const dim3 grid(n_segments, s.heads, (s.vdim + block_cols - 1) / block_cols);
+    const dim3 grid(n_segments, s.heads, shape.column_blocks);
     const int group = s.heads * s.dim % 4 == 0 && s.heads * s.vdim % 4 == 0 ? 4 : 1;       // channels a thread of the channel kernel
     const int per_block = kChannelThreads * group;
     const dim3 channel_grid((rows + kChannelRows - 1) / kChannelRows,
                             (s.heads * s.dim + per_block - 1) / per_block + (s.gate_rank ? (s.heads * s.vdim + per_block - 1) / per_block : 0));
     const size_t channel_shared = sizeof(float) * kChannelRows * (static_cast<size_t>(s.decay_rank > s.gate_rank ? s.decay_rank : s.gate_rank) + per_block);
-    // Pieces where whole segments leave the SMs short of blocks: up to eight blocks an SM, and at least six pieces (the two passes take
-    // the time of two pieces, and pieces slow one another).  Measured at 2048 rows of 128 x 128: 64 blocks in 16 pieces 270 -> 150 us,
-    // 128 blocks (two requests) in 9 pieces 281 -> 235 us; 256 blocks in 4 pieces 433 -> 580 us.
-    WalkPieces pieces = {ends, 1};
-    if (ends && s.rule != 1 && fixed_size) {
-        const long long blocks = static_cast<long long>(n_segments) * grid.y * grid.z;
-        const long long most = std::min(std::min(8ll * mlr_sm_count() / blocks, static_cast<long long>(rows / n_segments / kLeastPiece)), 16ll);
-        if (most >= 6) pieces.most = static_cast<int>(most);
-    }
+    const WalkPieces pieces = {ends, ends ? shape.pieces : 1};
 #define MLR_PASS(T, DIM, RULE, CH, NC, PASS)                                                                                           \
     do {                                                                                                                               \
         const auto kernel = recurrence_scan16_kernel<T, DIM, RULE, CH, NC, PASS>;                                                      \

@@ -22,6 +22,7 @@ import torch
 from ..config.base import ConfigError
 from ..config.registry import register_part
 from ..ops import functions as F
+from ..ops import native
 from ..ops.specs import GATES, RecurrenceSpec, address
 from ..weights.loader import WeightSpec
 from .base import RunContext, SequenceCore, StateNeed, columns_of
@@ -58,8 +59,9 @@ def emit_recurrence(b, mixer, proj, side, act, run: RunContext) -> None:
     kf = b.temp(proj.rows, d.qk_heads * d.dim, torch.float32)
     gates = b.temp(proj.rows, 2 * d.heads, torch.float32)
     obuf = b.temp(proj.rows, d.heads * d.vdim, torch.float32)
-    # Room for the ends of a walk's pieces (a place per 128 rows): rules whose pieces can run side by side.
-    ends = b.temp(proj.rows, -(-d.heads * (d.vdim + 1) * d.dim // 128), torch.float32) if d.rule != 1 else None
+    # Room for the ends of a walk's pieces, where steps of this many rows can be walked in pieces.
+    places = native.module("recurrence").mlr_linear_recurrence_places(address(d), b.bound(proj.rows))
+    ends = b.temp(places, d.heads * (d.vdim + 1) * d.dim, torch.float32) if places else None
     b.launch("recurrence", "mlr_linear_recurrence_pieces", address(d), proj.ptr, proj.ld, side.ptr, side.ld, proj.is_bf16, act.ptr,
              act.ld, state.data_ptr(), state.stride(0), info, b.segments, b.meta("positions"), proj.rows, qf.ptr, kf.ptr, gates.ptr,
              obuf.ptr, df.ptr if df else None, gf.ptr if gf else None, made, ends.ptr if ends else None, b.stream)

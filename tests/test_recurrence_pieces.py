@@ -99,3 +99,36 @@ def test_the_second_pass_leaves_the_ends_alone():
         place = int(off.nan_to_num(float("inf")).argmin())
         assert float(off[place]) <= 1e-5 * float(want.abs().max())
         assert torch.allclose(ends[place, :, vdim], (decay ** length)[:, None].expand(heads, dim), rtol=1e-4)
+
+
+@pytest.mark.parametrize("rule,dim,vdim,heads,segments,pieces", [("decay", 128, 128, 8, [2048], 16), ("decay", 128, 128, 8, [900, 1400], 8), ("step", 128, 64, 40, [900], 7),
+                                                                 ("decay", 64, 16, 2, [800] * 9, 6), ("step", 128, 64, 128, [8192], 1),
+                                                                 ("decay", 128, 128, 8, [767], 1), ("decay", 48, 16, 1, [2048], 1), ("delta", 128, 128, 2, [2048], 1)])
+def test_room_for_the_ends_is_what_the_walk_uses(rule, dim, vdim, heads, segments, pieces):
+    """Room is asked for where a step of these rows can be walked in pieces, bounded by the pieces that are launched, not by the rows."""
+    from mini_llm_runtime_b200.ops import native
+    g, rows, value = torch.Generator().manual_seed(dim + heads), sum(segments), heads * (vdim + 1) * dim
+    draw = lambda *shape: torch.randn(*shape, generator=g).cuda()
+    ca = 2 * heads * dim + heads * vdim
+    decay, a_log, dt_bias = torch.full((heads,), 0.99, device="cuda"), draw(heads), draw(heads)
+    spec = RecurrenceSpec(decay=decay.data_ptr(), a_log=a_log.data_ptr(), dt_bias=dt_bias.data_ptr(), skip=dt_bias.data_ptr(), heads=heads, qk_heads=heads,
+                          dim=dim, vdim=vdim, rule=RecurrenceSpec.RULE[rule], gate_first=int(rule == "step"), norm_parts=heads, col_k=heads * dim,
+                          col_v=2 * heads * dim, col_a=ca, col_b=ca + heads, q_mult=dim ** -0.5, k_mult=dim ** -0.5, unit_eps=1e-6, eps=1e-5, out_scale=1.0)
+    places = native.module("recurrence").mlr_linear_recurrence_places(ctypes.addressof(spec), rows)
+    if pieces == 1:
+        assert places == 0
+        return
+    assert len(segments) * pieces <= places <= 8 * 148
+    proj, ends = draw(rows, ca + 2 * heads), torch.full((places + 1, value), float("nan"), device="cuda")
+    first, info = 0, []
+    for i, n in enumerate(segments):
+        info.append((first, n, 0, i))
+        first += n
+    info = torch.tensor(info, dtype=torch.int32, device="cuda")
+    state, out, obuf = torch.zeros(len(segments), heads * vdim * dim, device="cuda"), torch.empty(rows, heads * vdim, device="cuda"), torch.empty(rows, heads * vdim, device="cuda")
+    q, k, gates, positions = draw(rows, heads * dim), draw(rows, heads * dim), draw(rows, 2 * heads), torch.zeros(rows, dtype=torch.int32, device="cuda")
+    _call("mlr_linear_recurrence_pieces", ctypes.addressof(spec), proj.data_ptr(), proj.stride(0), proj.data_ptr(), proj.stride(0), 0, out.data_ptr(),
+          out.stride(0), state.data_ptr(), state.stride(0), info.data_ptr(), len(segments), positions.data_ptr(), rows, q.data_ptr(), k.data_ptr(),
+          gates.data_ptr(), obuf.data_ptr(), None, None, 0, ends.data_ptr(), _stream())
+    used = torch.isfinite(ends).any(1).nonzero().flatten().tolist()
+    assert used and max(used) < len(segments) * pieces

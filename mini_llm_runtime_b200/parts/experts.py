@@ -132,12 +132,12 @@ class RoutedExperts(FeedForward):
         # A decode step's few rows are a pass over the chosen experts' weights.
         few = bool(both) and b.le(rows, 8)
         if grouped:
-            side = b.temp(rows, top * self.width, rt.dtype)        # the rows of the first product side by side
-            b.launch("experts", "mlr_experts_gather", x.ptr, x.ld, pair_of_row.ptr, rows, top, first_row.ptr, E, side.ptr, self.width, b.stream)
+            # The rows of the first product side by side, in the memory that the second product's result takes once they are used up.
+            b.launch("experts", "mlr_experts_gather", x.ptr, x.ld, pair_of_row.ptr, rows, top, first_row.ptr, E, y.ptr, self.width, b.stream)
 
         def product(a, lda, source, divisor, w, w2, kind, N, K, out, out_f32, shape):
             if grouped:
-                b.launch("gemm_bf16_tcgen05_pair", "mlr_grouped_product_bf16", side.ptr if source is not None else a, K, rows, top, w, w2, E, kind, N, K, out, N,
+                b.launch("gemm_bf16_tcgen05_pair", "mlr_grouped_product_bf16", y.ptr if source is not None else a, K, rows, top, w, w2, E, kind, N, K, out, N,
                          tiles.ptr, n_tiles.ptr, *shape, b.status, b.stream)
             elif few and a % 16 == 0 and lib.mlr_experts_few(K, lda):
                 b.launch("experts", "mlr_experts_product_few", a, lda, source, divisor, w, w2, kind, N, K, out, N, tiles.ptr, n_tiles.ptr, rows, top,

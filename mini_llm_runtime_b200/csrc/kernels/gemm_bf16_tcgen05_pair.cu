@@ -195,6 +195,7 @@ __global__ void __launch_bounds__(kThreads) gemm_tcgen05_pair_kernel(const __gri
 #pragma unroll 2
                 for (int c = 0; c < kTileN / 2; c += 16) {
                     uint32_t g[16], u[16];
+                    __syncwarp();           // the load takes the whole warp, rows past the tile's last one included
                     tmem_load16(row_base + c, g);
                     tmem_load16(row_base + kTileN / 2 + c, u);
                     if (p >= p_end) continue;
@@ -222,6 +223,7 @@ __global__ void __launch_bounds__(kThreads) gemm_tcgen05_pair_kernel(const __gri
 #pragma unroll 2
                 for (int c = 0; c < kTileN / 2; c += 16) {
                     uint32_t g[16], u[16];
+                    __syncwarp();           // as above
                     tmem_load16(row_base + c, g);
                     tmem_load16(row_base + kTileN / 2 + c, u);
                     if (p < P) {
@@ -254,6 +256,7 @@ __global__ void __launch_bounds__(kThreads) gemm_tcgen05_pair_kernel(const __gri
 #pragma unroll 4
                 for (int c = 0; c < kTileN; c += 16) {
                     uint32_t r[16];
+                    __syncwarp();           // as above
                     tmem_load16(row_base + c, r);
                     if (p >= p_end) continue;
                     const bool whole = q0 + c + 16 <= Q && (ldo & 7) == 0;

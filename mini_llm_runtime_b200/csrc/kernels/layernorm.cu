@@ -21,7 +21,6 @@ __global__ void __launch_bounds__(kThreads) depth_norm_kernel(float* h, const fl
                                                               const float* bias, float* history, long long slot_stride, int n_prev,
                                                               const float* dwa, const float* norm_w, const float* norm_b, float eps,
                                                               TO* out, long long ld_out, const int* want_rows, int width, int store_h) {
-    mlr_grid_dependents_may_start();
     mlr_grid_wait();
     extern __shared__ __align__(16) float xs[];       // [width]
     __shared__ float scratch[32];
@@ -110,6 +109,7 @@ __global__ void __launch_bounds__(kThreads) depth_norm_kernel(float* h, const fl
             sum += v;
         }
     }
+    mlr_grid_dependents_may_start();     // only now: waiting blocks of the next grid take room that this one's need
     if (!out) return;
     const float mean = mlr_block_sum(sum, scratch) / static_cast<float>(width);
     float squares = 0.0f;

@@ -61,7 +61,6 @@ __global__ void __launch_bounds__(kThreads) group_rmsnorm_kernel(float* h, const
                                                                  const int* rows, int width, int groups, float eps, int mode, float h_mult, Pieces pieces) {
     const int norm_delta = mode & 5, plain_out = mode & 2, norm_sum = mode & 4;
     __shared__ StagedPieces staged;
-    mlr_grid_dependents_may_start();
     mlr_grid_wait();
     extern __shared__ __align__(16) unsigned char smem[];
     float* vals = reinterpret_cast<float*>(smem);
@@ -136,6 +135,7 @@ __global__ void __launch_bounds__(kThreads) group_rmsnorm_kernel(float* h, const
             if constexpr (VEC) store4(o, i, kept(i));
             else mlr_store(o, i, vals[i]);
         }
+        mlr_grid_dependents_may_start();
         return;
     }
     __syncthreads();
@@ -152,6 +152,7 @@ __global__ void __launch_bounds__(kThreads) group_rmsnorm_kernel(float* h, const
         if constexpr (VEC) store4(o, i, v);
         else mlr_store(o, i, v.x);
     }
+    mlr_grid_dependents_may_start();     // only now: waiting blocks of the next grid take room that this one's need
 }
 
 // The same for rows of at most NQ * 1024 columns that can be read four at a time, in groups of a multiple of 128 columns: a thread

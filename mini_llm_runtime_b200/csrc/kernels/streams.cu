@@ -29,11 +29,12 @@ struct StreamWeights {
 
 // S: the number of copies when it is at most 8 (weights in registers, loops unrolled), or 0 for any number up to kMaxStreams
 // (weights in shared memory).  V: columns a thread takes at a time (4 when the width and all strides allow 16-byte accesses).
+// The next launch may start when the row is done: earlier, its waiting blocks take room that this one's need (300 rows of 8192: 9.6 us, at
+// the end 8.1 us).
 template <typename TO, int S, int V>
 __global__ void __launch_bounds__(kThreads) streams_step_kernel(float* h, const float* y, long long ld_y, const float* y_scale, const float* mix,
                                                                  const float* w_out, const float* w_in, const float* norm_weight, float eps,
                                                                  TO* out, long long ld_out, const int* rows, int width, int streams_given, Pieces pieces) {
-    mlr_grid_dependents_may_start();
     mlr_grid_wait();
     __shared__ StagedPieces staged;
     extern __shared__ __align__(16) float u[];          // [width]
@@ -135,7 +136,10 @@ __global__ void __launch_bounds__(kThreads) streams_step_kernel(float* h, const 
             }
         }
     }
-    if (!out) return;
+    if (!out) {
+        mlr_grid_dependents_may_start();
+        return;
+    }
     const float inv = 1.0f / sqrtf(mlr_block_sum(squares, scratch) / static_cast<float>(width) + eps);
     TO* orow = out + static_cast<size_t>(blockIdx.x) * ld_out;
     for (int c = threadIdx.x * V; c < width; c += kThreads * V) {         // a thread's own columns
@@ -145,6 +149,7 @@ __global__ void __launch_bounds__(kThreads) streams_step_kernel(float* h, const 
         for (int e = 0; e < V; ++e) value[e] = u[c + e] * inv * (norm_weight ? weight[e] : 1.0f);
         mlr_store_group<V>(orow + c, value);
     }
+    mlr_grid_dependents_may_start();
 }
 
 // The same for 1 to 4 copies of at most NQ * 1024 columns, four at a time: a thread keeps its columns in registers and asks for

@@ -155,20 +155,20 @@ __global__ void __launch_bounds__(kThreads) group_rmsnorm_kernel(float* h, const
     mlr_grid_dependents_may_start();     // only now: waiting blocks of the next grid take room that this one's need
 }
 
-// The same for rows of at most NQ * 1024 columns that can be read four at a time, in groups of a multiple of 128 columns: a thread
+// The same for rows of at most NQ * 4 * THREADS columns that can be read four at a time, in groups of a multiple of 128 columns: a thread
 // keeps its NQ groups of four columns in registers from the first load to the last store, and its loads are on their way
 // together.  A warp's 128 neighbouring columns are one chunk of one group; a chunk is summed by its warp, a group's chunks in
 // order.  The kernel above stages the row in shared memory and goes back to memory for every group of columns, which the
-// few rows of a decode step pay in full: two rows of 2048 in four groups 5.1 -> 4.9 us, and the next launch starts meanwhile.
-template <typename T, int NQ>
-__global__ void __launch_bounds__(kThreads) group_rmsnorm_quads_kernel(float* h, const float* delta, int ld_delta, const float* bias,
+// few rows of a decode step pay in full: three rows of 2048 in four groups 4.0 -> 2.8 us, of 4096 in 32 groups 7.9 -> 3.5 us.
+template <typename T, int NQ, int THREADS>
+__global__ void __launch_bounds__(THREADS) group_rmsnorm_quads_kernel(float* h, const float* delta, int ld_delta, const float* bias,
                                                                        const float* w_post, const float* w_pre, T* out, int ld_out,
                                                                        const int* rows, int width, int groups, float eps, int mode, float h_mult,
                                                                        Pieces pieces) {
     const int norm_delta = mode & 5, plain_out = mode & 2, norm_sum = mode & 4;
-    constexpr int kStep = kThreads * 4;
+    constexpr int kStep = THREADS * 4, kWarps = THREADS / 32;
     __shared__ StagedPieces staged;
-    __shared__ float chunk_sums[NQ * kThreads / 32];
+    __shared__ float chunk_sums[NQ * kWarps];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int i0 = threadIdx.x * 4, part = width / groups, per_group = part / 128;
     const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -184,20 +184,26 @@ __global__ void __launch_bounds__(kThreads) group_rmsnorm_quads_kernel(float* h,
 #pragma unroll
         for (int k = 0; k < NQ; ++k) {
             const float sum = mlr_warp_sum(fmaf(v[k].w, v[k].w, fmaf(v[k].z, v[k].z, fmaf(v[k].y, v[k].y, v[k].x * v[k].x))));
-            if (lane == 0) chunk_sums[k * (kThreads / 32) + warp] = sum;
+            if (lane == 0) chunk_sums[k * kWarps + warp] = sum;
         }
         __syncthreads();
+        // One group: every warp adds its chunks, lanes side by side.  More: lane k has the group of the warp's k-th chunk (the whole warp for one chunk
+        // after the other cost 2048 rows of 4096 in 32 groups 47 us, so 26 us).
+        if (groups == 1) {
+            float total = 0.0f;
+            for (int c = lane; c < per_group; c += 32) total += chunk_sums[c];
+            inv_rms = 1.0f / sqrtf(mlr_warp_sum(total) / static_cast<float>(part) + eps);
+        } else if (lane < NQ && (lane * kWarps + warp) * 128 < width) {
+            const float* first = chunk_sums + (lane * kWarps + warp) / per_group * per_group;
+            float total = 0.0f;
+            for (int c = 0; c < per_group; ++c) total += first[c];
+            inv_rms = 1.0f / sqrtf(total / static_cast<float>(part) + eps);
+        }
 #pragma unroll
         for (int k = 0; k < NQ; ++k) {
-            const int first = groups == 1 ? 0 : (k * (kThreads / 32) + warp) / per_group * per_group;
+            const float inv = groups == 1 ? inv_rms : __shfl_sync(0xffffffffu, inv_rms, k);
             if (i0 + k * kStep >= width) continue;        // (whole warps)
-            if (k == 0 || groups > 1) {
-                float total = 0.0f;
-                for (int c = lane; c < per_group; c += 32) total += chunk_sums[first + c];
-                total = mlr_warp_sum(total);
-                inv_rms = 1.0f / sqrtf(total / static_cast<float>(part) + eps);
-            }
-            v[k].x *= inv_rms; v[k].y *= inv_rms; v[k].z *= inv_rms; v[k].w *= inv_rms;
+            v[k].x *= inv; v[k].y *= inv; v[k].z *= inv; v[k].w *= inv;
             if (w) { v[k].x *= weight[k].x; v[k].y *= weight[k].y; v[k].z *= weight[k].z; v[k].w *= weight[k].w; }
         }
     };
@@ -274,18 +280,18 @@ int group_rmsnorm(float* h, const float* delta, int ld_delta, const float* bias,
     const auto aligned = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
     const bool vec = width % 4 == 0 && ld_delta % 4 == 0 && ld_out % 4 == 0 && aligned(h) && aligned(delta) && aligned(bias) && aligned(w_post) &&
                      aligned(w_pre) && aligned(out) && (!pieces.y || pieces_aligned(pieces));
-    // In registers where four columns go at once and a group is whole chunks of 128 (the row's width decides, not the number of rows).
-    const bool quads = vec && width / groups % 128 == 0 && width <= 8 * 4 * kThreads;
-#define MLR_QUADS(T, NQ)                                                                                                               \
-    mlr_launch((group_rmsnorm_quads_kernel<T, NQ>), dim3(count), dim3(kThreads), 0, stream, h, delta, ld_delta, bias, w_post, w_pre,    \
-               static_cast<T*>(out), ld_out, rows, width, groups, eps, norm_delta, h_mult, pieces)
-#define MLR_PICK(T)                                     \
-    do {                                                \
-        const int per = (width + 4 * kThreads - 1) / (4 * kThreads); \
-        if (per <= 1) MLR_QUADS(T, 1);                  \
-        else if (per <= 2) MLR_QUADS(T, 2);             \
-        else if (per <= 4) MLR_QUADS(T, 4);             \
-        else MLR_QUADS(T, 8);                           \
+    // In registers where four columns go at once and a group is whole chunks of 128 (the row's width decides, not the number of rows).  Rows of more than
+    // 4096 columns stay above: with eight groups of four a thread 2048 rows of 8192 take 84 us, there 61 us.
+    const bool quads = vec && width / groups % 128 == 0 && width <= 16 * kThreads;
+#define MLR_QUADS(T, NQ, THREADS)                                                                                                      \
+    mlr_launch((group_rmsnorm_quads_kernel<T, NQ, THREADS>), dim3(count), dim3(THREADS), 0, stream, h, delta, ld_delta, bias, w_post,   \
+               w_pre, static_cast<T*>(out), ld_out, rows, width, groups, eps, norm_delta, h_mult, pieces)
+#define MLR_PICK(T)                                                                      \
+    do {                                                                                 \
+        if (width <= 4 * kThreads) MLR_QUADS(T, 1, kThreads);                            \
+        else if (width <= 8 * kThreads && pieces.y) MLR_QUADS(T, 1, 2 * kThreads);       \
+        else if (width <= 8 * kThreads) MLR_QUADS(T, 2, kThreads);                       \
+        else MLR_QUADS(T, 4, kThreads);                                                  \
     } while (0)
     if (quads) {
         if (out_bf16) MLR_PICK(__nv_bfloat16);

@@ -70,7 +70,7 @@ def test_depth_average_and_layer_norm(dtype, width, states):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("width,states,off,gap", [(16388, 1, 0, 0), (20480, 6, 0, 0), (2048, 3, 1, 0), (4100, 5, 2, 0), (1030, 2, 0, 0), (1024, 4, 0, 2)])
+@pytest.mark.parametrize("width,states,off,gap", [(16388, 1, 0, 0), (20480, 6, 0, 0), (2048, 3, 1, 0), (4100, 5, 2, 0), (1030, 2, 0, 0), (1024, 4, 0, 2), (1028, 5, 0, 0), (2048, 0, 0, 0)])
 def test_depth_average_and_layer_norm_of_other_rows(dtype, width, states, off, gap):
     """Rows wider than a thread's registers take, results and norm weights `off` a border, results to add whose rows lie `gap` off one."""
     from mini_llm_runtime_b200.ops import native
@@ -142,3 +142,65 @@ def test_copies_of_the_stream(dtype, streams, width):
     _near(h.view(rows, streams, width), new, torch.float32)
     read = (new * w_in.double()[None, :, None]).sum(1)
     _near(out, _grouped(read, 1, 1e-5) * norm_w.double(), dtype)
+
+
+def _pieces(draw, rows, top, width, x_dtype):
+    """What routed experts leave of a token: pieces (one of them an identity expert's, without a row), a gated shared result, the token
+    itself for its identity experts.  The kernels' arguments and the sum in 64 bits."""
+    y, weights, shared, gate, passed = draw(rows * top, width), draw(rows, top), draw(rows, width), draw(rows), draw(rows)
+    x = draw(rows, width).to(x_dtype)
+    place = torch.randperm(rows * top, generator=torch.Generator().manual_seed(2)).to(torch.int32).view(rows, top).cuda()
+    place[0, 1] = place[2, 0] = -1
+    total = ((weights.double() * (place >= 0))[:, :, None] * y.double()[place.clamp(min=0).long()]).sum(1)
+    total = total + gate.double()[:, None] * shared.double() + passed.double()[:, None] * x.double()
+    args = (y.data_ptr(), width, place.data_ptr(), weights.data_ptr(), top, shared.data_ptr(), width, gate.data_ptr(), x.data_ptr(), width,
+            int(x_dtype is torch.bfloat16), passed.data_ptr())
+    return args, total, (y, weights, shared, gate, passed, x, place)
+
+
+@pytest.mark.parametrize("x_dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("width,groups", [(1024, 1), (2048, 2), (3200, 5), (4096, 32), (8192, 8), (1000, 4)])
+def test_grouped_norm_of_pieces_with_identity_experts(x_dtype, width, groups):
+    from mini_llm_runtime_b200.ops import native
+    draw, rows, top = _draw(width + groups), 3, 5
+    h, w_post, w_pre = draw(rows, width), draw(width), draw(width)
+    args, total, held = _pieces(draw, rows, top, width, x_dtype)
+    out, old = torch.empty(rows, width, device="cuda"), h.double()
+    _call("norm_grouped", "mlr_group_rmsnorm_pieces", h.data_ptr(), *args, w_post.data_ptr(), w_pre.data_ptr(), out.data_ptr(), width, 0, rows, width,
+          groups, 1e-5, 1, native.stream())
+    stream = old + _grouped(total, groups, 1e-5) * w_post.double()
+    _near(h, stream, torch.float32)
+    _near(out, _grouped(stream, groups, 1e-5) * w_pre.double(), torch.float32)
+
+
+@pytest.mark.parametrize("x_dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("streams,width,reads", [(1, 4096, True), (2, 1028, True), (4, 2048, False), (4, 4096, True), (3, 4096, False), (2, 8192, True)])
+def test_copies_of_the_stream_take_pieces(x_dtype, streams, width, reads):
+    """With and without a norm behind the sub-layer."""
+    from mini_llm_runtime_b200.ops import native
+    draw, rows, top = _draw(streams + width + reads), 3, 5
+    h, scale, norm_w = draw(rows, streams * width), draw(width), draw(width)
+    mix, w_out, w_in = draw(streams, streams), draw(streams), draw(streams)
+    args, total, held = _pieces(draw, rows, top, width, x_dtype)
+    out, old = torch.empty(rows, width, device="cuda"), h.double().view(rows, streams, width)
+    _call("streams", "mlr_streams_step_pieces", h.data_ptr(), *args, scale.data_ptr(), mix.data_ptr(), w_out.data_ptr(), w_in.data_ptr(), norm_w.data_ptr(),
+          1e-5, out.data_ptr() if reads else None, width, 0, rows, width, streams, native.stream())
+    new = torch.einsum("rsw,st->rtw", old, mix.double()) + w_out.double()[None, :, None] * (total * scale.double())[:, None]
+    _near(h.view(rows, streams, width), new, torch.float32)
+    if reads:
+        _near(out, _grouped((new * w_in.double()[None, :, None]).sum(1), 1, 1e-5) * norm_w.double(), torch.float32)
+
+
+@pytest.mark.parametrize("streams,width", [(1, 1024), (4, 2048), (4, 4096)])
+def test_copies_of_the_stream_of_wanted_rows(streams, width):
+    """A launch over some rows norms what it reads of them and writes nothing back."""
+    from mini_llm_runtime_b200.ops import native
+    draw = _draw(streams + width)
+    h, w_in, norm_w = draw(6, streams * width), draw(streams), draw(width)
+    rows = torch.tensor([4, 0, 5], dtype=torch.int32, device="cuda")
+    out, before = torch.empty(3, width, device="cuda"), h.clone()
+    _call("streams", "mlr_streams_step", h.data_ptr(), None, 0, None, None, None, w_in.data_ptr(), norm_w.data_ptr(), 1e-5, out.data_ptr(), width, 0,
+          rows.data_ptr(), 3, width, streams, native.stream())
+    read = (h.double().view(6, streams, width)[rows.long()] * w_in.double()[None, :, None]).sum(1)
+    _near(out, _grouped(read, 1, 1e-5) * norm_w.double(), torch.float32)
+    assert torch.equal(h, before)

@@ -97,7 +97,7 @@ __global__ void rmsnorm_kernel(float* __restrict__ h, const float* __restrict__ 
 // The same for widths that are multiples of 4 and fit 16 values per thread of the `owners` (a power of two of threads that depends
 // on the width alone): values stay in registers between the two passes, so the row is read once and every load of the
 // row is in flight at the same time.  One block per row.  QUADS 4: a block is the owners, a thread loads its four groups of
-// four values; QUADS 1: four threads stand for an owner.  The sums are the same: four values in a chain, an owner's four
+// four values; QUADS 2 and 1: two or four threads stand for an owner.  The sums are the same: four values in a chain, an owner's four
 // groups as (0 + 1) + (2 + 3), then a fixed tree over the owners.
 template <typename T, typename W, int QUADS>
 __global__ void __launch_bounds__(1024) rmsnorm_cached_kernel(float* __restrict__ h, const float* __restrict__ delta,
@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(1024) rmsnorm_cached_kernel(float* __restrict_
     mlr_grid_dependents_may_start();
     mlr_grid_wait();
     __shared__ float scratch[32];
-    __shared__ float groups[QUADS == 1 ? 1024 : 1];
+    __shared__ float groups[QUADS == 1 ? 1024 : QUADS == 2 ? 2048 : 1];       // by group of four values
     const int r = blockIdx.x;
     const size_t row = rows ? static_cast<size_t>(rows[r]) : static_cast<size_t>(r);
     float4* hr = reinterpret_cast<float4*>(h + row * width);
@@ -136,8 +136,9 @@ __global__ void __launch_bounds__(1024) rmsnorm_cached_kernel(float* __restrict_
 #pragma unroll
     for (int k = 0; k < QUADS; ++k) sums[k] = fmaf(x[k].w, x[k].w, fmaf(x[k].z, x[k].z, fmaf(x[k].y, x[k].y, x[k].x * x[k].x)));
     float sum;
-    if constexpr (QUADS == 1) {
-        groups[threadIdx.x] = sums[0];
+    if constexpr (QUADS < 4) {
+#pragma unroll
+        for (int k = 0; k < QUADS; ++k) groups[threadIdx.x + k * blockDim.x] = sums[k];
         __syncthreads();
         const int owner = threadIdx.x & (owners - 1);
         sum = (groups[owner] + groups[owner + owners]) + (groups[owner + 2 * owners] + groups[owner + 3 * owners]);
@@ -551,23 +552,26 @@ MLR_API int mlr_rmsnorm(float* h, const float* delta, int slices, long long slic
     MLR_REQUIRE(eps > 0.0f, "rmsnorm: eps must be positive, got %g", static_cast<double>(eps));
     if (count == 0) return 0;
     const int threads = row_threads(width);
-    // Register-cached path: width a multiple of 4, at most 16 values per thread of a block
-    // of up to 1024 threads, 16-byte aligned rows.  A thread takes 16 values where the rows outnumber the SMs: its four loads are
-    // on their way together and several blocks share an SM.  With four values a thread a row of 4096 is one block of 1024
-    // threads an SM (registers), which waits for memory and for its own sum with nothing beside it: 2048 rows of 4096
-    // 34 us, with 256 threads a row 14 us.  Rows that have an SM each are better off with more threads (the 8B decode step of 40
-    // rows: 5.51 ms with 256 threads a row, 5.40 ms with 1024).
-    int cached_threads = 64;
+    // Register-cached path: width a multiple of 4, at most 16 values per thread of a block of up to 1024 threads, 16-byte aligned rows.
+    // While the rows' blocks fit the SMs in one round a row takes as many threads an owner as it has groups of four values for: it is bound by its
+    // own waits (the 8B decode step of 40 rows: 5.51 ms with 256 threads a row, 5.40 ms with 1024; 300 rows of 1024 3.1 us with 64, 2.2 us
+    // with 256; 40 rows of 8192 3.5 us with 512, 3.0 us with 1024).  Beyond, a thread takes an owner's 16 values: its four loads are on their way
+    // together and more rows share an SM.  With four values a thread a row of 4096 is one block of 1024 threads an SM, which waits for
+    // memory and for its own sum with nothing beside it: 2048 rows of 4096 24 us, with 256 threads a row 10 us.
+    int cached_threads = 32;
     while (cached_threads < 1024 && cached_threads * 16 < width) cached_threads <<= 1;
-    const bool spread = cached_threads <= 256 && count <= mlr_sm_count();
+    int spread = cached_threads > 512 ? 1 : cached_threads > 256 ? 2 : 4;
+    while (spread > 1 && spread / 2 * cached_threads * 4 >= width) spread /= 2;
+    const int block = spread * cached_threads, at_once = block > 512 ? 1 : block > 256 ? 3 : 2048 / block;       // blocks of that many threads an SM
+    if (count > mlr_sm_count() * at_once) spread = 1;
     const bool cached = width % 4 == 0 && width <= cached_threads * 16 && reinterpret_cast<uintptr_t>(h) % 16 == 0 &&
                         (!delta || (reinterpret_cast<uintptr_t>(delta) % 16 == 0 && slice_stride % 4 == 0)) &&
                         reinterpret_cast<uintptr_t>(out) % 16 == 0 && reinterpret_cast<uintptr_t>(weight) % 16 == 0;
 #define MLR_LAUNCH(T, W)                                                                                   \
     do {                                                                                                   \
         if (cached)                                                                                        \
-            mlr_launch((spread ? rmsnorm_cached_kernel<T, W, 1> : rmsnorm_cached_kernel<T, W, 4>), dim3(count), \
-                dim3(spread ? 4 * cached_threads : cached_threads), 0, stream,                             \
+            mlr_launch((spread == 4 ? rmsnorm_cached_kernel<T, W, 1> : spread == 2 ? rmsnorm_cached_kernel<T, W, 2> : rmsnorm_cached_kernel<T, W, 4>), \
+                dim3(count), dim3(spread * cached_threads), 0, stream,                             \
                 h, delta, slices, static_cast<size_t>(slice_stride), static_cast<const W*>(weight),       \
                 static_cast<T*>(out), rows, width, eps, write_back, cached_threads);                       \
         else                                                                                               \

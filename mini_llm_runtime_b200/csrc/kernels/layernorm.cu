@@ -132,8 +132,9 @@ __global__ void __launch_bounds__(kThreads) depth_norm_kernel(float* h, const fl
 // which one row of a decode step pays in full.  Measured with rows of 4096 in a step: one row 14.8 -> 4.8 us, 2048 rows 47 -> 40 us.
 constexpr int kQuads = 4;
 
-// THREADS: the most a block has (what it leaves each thread in registers).
-template <typename TO, int THREADS>
+// NQ: a thread's groups of four columns.  THREADS: the most a block has (what it leaves each thread in registers).  Rows of up to 2048 columns have a
+// thread for every group: empty groups cost their registers and instructions (2048 rows of 512 with four states 17.2 us with four).
+template <typename TO, int NQ, int THREADS>
 __global__ void __launch_bounds__(THREADS) depth_norm_quads_kernel(float* h, const float* d1, long long ld1, const float* d2, long long ld2,
                                                                 const float* bias, float* history, long long slot_stride, int n_prev,
                                                                 const float* dwa, const float* norm_w, const float* norm_b, float eps,
@@ -146,27 +147,27 @@ __global__ void __launch_bounds__(THREADS) depth_norm_quads_kernel(float* h, con
     float* hrow = h + static_cast<size_t>(row) * width;
     const int c0 = threadIdx.x * 4, step = blockDim.x * 4;
     const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    auto load = [&](const float* p, float4 (&v)[kQuads]) {
+    auto load = [&](const float* p, float4 (&v)[NQ]) {
 #pragma unroll
-        for (int k = 0; k < kQuads; ++k) v[k] = c0 + k * step < width ? __ldcg(reinterpret_cast<const float4*>(p + c0 + k * step)) : zero;
+        for (int k = 0; k < NQ; ++k) v[k] = c0 + k * step < width ? __ldcg(reinterpret_cast<const float4*>(p + c0 + k * step)) : zero;
     };
-    auto store = [&](float* p, const float4 (&v)[kQuads]) {
+    auto store = [&](float* p, const float4 (&v)[NQ]) {
 #pragma unroll
-        for (int k = 0; k < kQuads; ++k)
+        for (int k = 0; k < NQ; ++k)
             if (c0 + k * step < width) *reinterpret_cast<float4*>(p + c0 + k * step) = v[k];
     };
-    auto plus = [](float4 (&v)[kQuads], const float4 (&a)[kQuads]) {
+    auto plus = [](float4 (&v)[NQ], const float4 (&a)[NQ]) {
 #pragma unroll
-        for (int k = 0; k < kQuads; ++k) { v[k].x += a[k].x; v[k].y += a[k].y; v[k].z += a[k].z; v[k].w += a[k].w; }
+        for (int k = 0; k < NQ; ++k) { v[k].x += a[k].x; v[k].y += a[k].y; v[k].z += a[k].z; v[k].w += a[k].w; }
     };
-    float4 x[kQuads];
+    float4 x[NQ];
     load(hrow, x);
     if (d1 || d2 || bias) {
-        float4 add[kQuads], more[kQuads];
+        float4 add[NQ], more[NQ];
         if (d1) load(d1 + static_cast<size_t>(row) * ld1, add);
         else {
 #pragma unroll
-            for (int k = 0; k < kQuads; ++k) add[k] = zero;
+            for (int k = 0; k < NQ; ++k) add[k] = zero;
         }
         if (d2) {
             load(d2 + static_cast<size_t>(row) * ld2, more);
@@ -180,40 +181,50 @@ __global__ void __launch_bounds__(THREADS) depth_norm_quads_kernel(float* h, con
     }
     if (history) {
         float* slot = history + static_cast<size_t>(row) * width;
-        float4 mixed[kQuads];
+        float4 mixed[NQ];
 #pragma unroll
-        for (int k = 0; k < kQuads; ++k) mixed[k] = zero;
-#pragma unroll 2
-        for (int j = 0; j < n_prev; ++j) {
-            float4 s[kQuads];
-            load(slot + static_cast<size_t>(j) * slot_stride, s);
-            const float w = dwa[j];
+        for (int k = 0; k < NQ; ++k) mixed[k] = zero;
+        auto mix = [&](float w, const float4 (&s)[NQ]) {
 #pragma unroll
-            for (int k = 0; k < kQuads; ++k) {
+            for (int k = 0; k < NQ; ++k) {
                 mixed[k].x = fmaf(w, s[k].x, mixed[k].x); mixed[k].y = fmaf(w, s[k].y, mixed[k].y);
                 mixed[k].z = fmaf(w, s[k].z, mixed[k].z); mixed[k].w = fmaf(w, s[k].w, mixed[k].w);
             }
+        };
+        constexpr int kAhead = NQ == 1 ? 4 : 2;             // states on their way at a time
+        int j = 0;
+        for (; j + kAhead <= n_prev; j += kAhead) {
+            float4 s[kAhead][NQ];
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u) load(slot + static_cast<size_t>(j + u) * slot_stride, s[u]);
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u) mix(dwa[j + u], s[u]);
+        }
+        for (; j < n_prev; ++j) {
+            float4 s[NQ];
+            load(slot + static_cast<size_t>(j) * slot_stride, s);
+            mix(dwa[j], s);
         }
         store(slot + static_cast<size_t>(n_prev) * slot_stride, x);
         const float w = dwa[n_prev];
 #pragma unroll
-        for (int k = 0; k < kQuads; ++k) {
+        for (int k = 0; k < NQ; ++k) {
             x[k].x = fmaf(w, x[k].x, mixed[k].x); x[k].y = fmaf(w, x[k].y, mixed[k].y);
             x[k].z = fmaf(w, x[k].z, mixed[k].z); x[k].w = fmaf(w, x[k].w, mixed[k].w);
         }
     }
     if (store_h) store(hrow, x);
     if (!out) return;
-    float4 weight[kQuads], shift[kQuads];
+    float4 weight[NQ], shift[NQ];
     load(norm_w, weight);
     if (norm_b) load(norm_b, shift);
     float sum = 0.0f;
 #pragma unroll
-    for (int k = 0; k < kQuads; ++k) sum += (x[k].x + x[k].y) + (x[k].z + x[k].w);      // columns past the row are zeros
+    for (int k = 0; k < NQ; ++k) sum += (x[k].x + x[k].y) + (x[k].z + x[k].w);      // columns past the row are zeros
     const float mean = mlr_block_sum(sum, scratch) / static_cast<float>(width);
     float squares = 0.0f;
 #pragma unroll
-    for (int k = 0; k < kQuads; ++k)
+    for (int k = 0; k < NQ; ++k)
         if (c0 + k * step < width) {
             x[k].x -= mean; x[k].y -= mean; x[k].z -= mean; x[k].w -= mean;
             squares = fmaf(x[k].x, x[k].x, squares); squares = fmaf(x[k].y, x[k].y, squares);
@@ -222,7 +233,7 @@ __global__ void __launch_bounds__(THREADS) depth_norm_quads_kernel(float* h, con
     const float inv = 1.0f / sqrtf(mlr_block_sum(squares, scratch) / static_cast<float>(width) + eps);
     TO* orow = out + static_cast<size_t>(r) * ld_out;
 #pragma unroll
-    for (int k = 0; k < kQuads; ++k)
+    for (int k = 0; k < NQ; ++k)
         if (c0 + k * step < width) {
             float4 v = make_float4(x[k].x * inv * weight[k].x, x[k].y * inv * weight[k].y, x[k].z * inv * weight[k].z, x[k].w * inv * weight[k].w);
             if (norm_b) { v.x += shift[k].x; v.y += shift[k].y; v.z += shift[k].z; v.w += shift[k].w; }
@@ -252,13 +263,17 @@ MLR_API int mlr_depth_norm(float* h, const float* d1, long long ld1, const float
     const auto fits = [](const void* p, size_t bytes) { return reinterpret_cast<uintptr_t>(p) % bytes == 0; };
     const bool quads = width % 4 == 0 && (n_prev == 0 || slot_stride >= width) && width <= 1024 * 4 * kQuads && ld1 % 4 == 0 && ld2 % 4 == 0 && slot_stride % 4 == 0 && ld_out % 4 == 0 &&
                        fits(out, out_bf16 ? 8 : 16) && fits(norm_w, 16) && fits(norm_b, 16);
-    int threads = kThreads;
+    int threads = 128;
+    while (threads < 2 * kThreads && threads * 4 < width) threads <<= 1;
+    if (width > 4 * threads) threads = kThreads;
     while (threads < 1024 && threads * 4 * kQuads < width) threads <<= 1;
 #define MLR_GO(TO)                                                                                                                         \
     do {                                                                                                                                   \
         if (quads) {                                                                                                                       \
-            mlr_launch((threads == kThreads ? depth_norm_quads_kernel<TO, kThreads> : depth_norm_quads_kernel<TO, 1024>), dim3(rows),      \
-                       dim3(threads), 0, stream, h, d1, ld1, d2, ld2, bias, history, slot_stride, n_prev, dwa, norm_w, norm_b, eps,        \
+            mlr_launch((threads <= 2 * kThreads && width <= 4 * threads ? depth_norm_quads_kernel<TO, 1, 2 * kThreads>                     \
+                        : threads == kThreads                           ? depth_norm_quads_kernel<TO, kQuads, kThreads>                    \
+                                                                        : depth_norm_quads_kernel<TO, kQuads, 1024>),                      \
+                       dim3(rows), dim3(threads), 0, stream, h, d1, ld1, d2, ld2, bias, history, slot_stride, n_prev, dwa, norm_w, norm_b, eps,        \
                        static_cast<TO*>(out), ld_out, want_rows, width, store_h);                                                          \
             break;                                                                                                                         \
         }                                                                                                                                  \

@@ -152,18 +152,18 @@ __global__ void __launch_bounds__(kThreads) streams_step_kernel(float* h, const 
     mlr_grid_dependents_may_start();
 }
 
-// The same for 1 to 4 copies of at most NQ * 1024 columns, four at a time: a thread keeps its columns in registers and asks for
+// The same for 1 to 4 copies of at most NQ * 4 * THREADS columns, four at a time: a thread keeps its columns in registers and asks for
 // all of them (every copy, the result or its pieces) before it uses the first.  The kernel above goes back to memory for every group of
 // columns, which the few rows of a decode step pay in full: one row of 4096 with pieces 10.2 -> 5.2 us, three rows of 4 x 2048 6.0 -> 4.4 us, 3863 rows of those 67 -> 60 us.
-template <typename TO, int S, int NQ>
-__global__ void __launch_bounds__(kThreads) streams_step_quads_kernel(float* h, const float* y, long long ld_y, const float* y_scale, const float* mix,
+template <typename TO, int S, int NQ, int THREADS>
+__global__ void __launch_bounds__(THREADS) streams_step_quads_kernel(float* h, const float* y, long long ld_y, const float* y_scale, const float* mix,
                                                                        const float* w_out, const float* w_in, const float* norm_weight, float eps,
                                                                        TO* out, long long ld_out, const int* rows, int width, Pieces pieces) {
     mlr_grid_dependents_may_start();
     mlr_grid_wait();
     __shared__ StagedPieces staged;
     __shared__ float scratch[32];
-    constexpr int kStep = kThreads * 4;
+    constexpr int kStep = THREADS * 4;
     const int row = rows ? rows[blockIdx.x] : blockIdx.x;
     const bool writes = y || pieces.y;
     const int c0 = threadIdx.x * 4;
@@ -306,16 +306,18 @@ int streams_step(float* h, const float* y, long long ld_y, const float* y_scale,
     const auto aligned = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
     const bool wide = width % 4 == 0 && aligned(h) && aligned(y) && ld_y % 4 == 0 && aligned(y_scale) && aligned(norm_weight) && aligned(out) &&
                       ld_out % 4 == 0 && (!pieces.y || pieces_aligned(pieces));
-    // A thread's columns in registers: up to 4 copies of up to 4096 columns (64 registers of stream).
+    // A thread's columns in registers: up to 4 copies of up to 4096 columns, at most 48 registers of stream (with 64 for four copies of 4096 one
+    // block of 256 threads fits where two do: 300 rows 9.8 us, in the kernel above 8.2 us).
     const bool quads = wide && streams <= 4 && width <= 4 * 4 * kThreads;
-#define MLR_QUADS(TO, S, NQ)                                                                                                               \
-    mlr_launch((streams_step_quads_kernel<TO, S, NQ>), dim3(count), dim3(kThreads), 0, stream, h, y, ld_y, y_scale, mix, w_out, w_in,        \
+#define MLR_QUADS(TO, S, NQ, THREADS)                                                                                                               \
+    mlr_launch((streams_step_quads_kernel<TO, S, NQ, THREADS>), dim3(count), dim3(THREADS), 0, stream, h, y, ld_y, y_scale, mix, w_out, w_in,        \
                norm_weight, eps, static_cast<TO*>(out), ld_out, rows, width, pieces)
 #define MLR_PER(TO, S)                                           \
     do {                                                         \
-        if (width <= 4 * kThreads) MLR_QUADS(TO, S, 1);          \
-        else if (width <= 8 * kThreads) MLR_QUADS(TO, S, 2);     \
-        else MLR_QUADS(TO, S, 4);                                \
+        if (width <= 4 * kThreads) MLR_QUADS(TO, S, 1, kThreads);                 \
+        else if (width <= 8 * kThreads) MLR_QUADS(TO, S, 2, kThreads);            \
+        else if (S < 4) MLR_QUADS(TO, S, 4, kThreads);                            \
+        else MLR_QUADS(TO, S, 2, 2 * kThreads);                                   \
     } while (0)
 #define MLR_COPIES(TO)                   \
     switch (streams) {                   \

@@ -34,7 +34,7 @@
 //    memory: a lane needs 16 bytes of its token's row per 512 values of K, eight registers' worth of loads, and
 //    shared memory is all ring (three slots at any row count).  A product that ADDS into the stream is cut along K
 //    into parts of at most 4096 values for that: each part adds its partial product into the stream (a cell has the
-//    same owner in every part).  So is one that stores float32: its first part stores, the others add (4096 x 12288
+//    same owner in every part).  So is one that stores float32 over more than 6144 values: its first part stores, the others add (4096 x 12288
 //    at one row: 20 us, against 65 us for 32 blocks of the one-block tcgen05 kernel).  Other products (a norm prologue, a wider K) stage their activations in shared
 //    memory beside a ring of two slots (three at one row), with shorter copies or one buffer of partial sums
 //    where room is short.
@@ -436,12 +436,18 @@ int slots_for(size_t x_bytes, int chunk) {
     return 2 * kPartialBytes + x_bytes + ring_bytes(chunk, kMostSlots) <= room ? kMostSlots : 2;
 }
 
-// How many parts a product over K values is cut into for M rows (1: it stays whole), and the width of a part.  Only a
-// product that adds into the stream or stores float32 can be cut; it is, when its activations would push the ring below its best size.
-// Whether a product keeps its activations in registers: its norm, if any, was prepared, and its K (or, for a product
-// that adds into the stream or stores float32, the K of its parts) is at most 512 * kRegisterBlocks.
-bool in_registers(int K, int mode, int norm) { return norm != 1 && (mode == kAddF32 || (mode == kStoreF32 && norm == 0) || K <= 512 * kRegisterBlocks); }
+// Whether a product keeps its activations in registers: its norm, if any, was prepared, and its K is at most 512 * kRegisterBlocks.  A product that
+// adds into the stream is cut along K into parts of that width; so is one that stores float32 over more than three chunks of K, or whose
+// activations do not fit shared memory whole.  (With up to three chunks the whole product is ahead, since a part's second chunk is partly empty:
+// 4096 x 5120 at one row 8.7 against 10.7 us, 1024 x 6144 4.8 against 5.8 us; 4096 x 8192 the other way, 13.7 against 11.9 us.  The most rows
+// decide about the room, so that a row's result does not depend on how many there are.)
+bool in_registers(int K, int mode, int norm) {
+    if (norm == 1) return false;
+    if (mode == kAddF32 || K <= 512 * kRegisterBlocks) return true;
+    return mode == kStoreF32 && norm == 0 && (K > 3 * kMostChunk || chunk_for(x_region_bytes(kMaxRows, K), 1) == 0);
+}
 
+// How many parts a product over K values is cut into for M rows (1: it stays whole), and the width of a part.
 int parts_of(int M, int K, int mode, int norm, int& part_width) {
     part_width = K;
     if (in_registers(K, mode, norm)) {

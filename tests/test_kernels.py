@@ -286,6 +286,18 @@ def test_gemv_bf16_stores_float32_of_a_wide_k_in_parts(M, N, K):
     assert torch.allclose(out.cpu().double(), x.double() @ w.double().T, atol=1e-4, rtol=1e-4)
 
 
+@pytest.mark.parametrize("N,K", [(40, 4104), (33, 5120), (24, 6144), (24, 6152), (17, 12288)])
+def test_gemv_bf16_float32_rows_have_the_bits_they_have_alone(N, K):
+    """Whole or in parts: the choice depends on K, not on the rows of the step."""
+    x, w = torch.randn(8, K, generator=gen(3)).to(torch.bfloat16).to(DEV), (torch.randn(N, K, generator=gen(4)) * K ** -0.5).to(torch.bfloat16).to(DEV)
+    out, alone = torch.full((8, N), float("nan"), device=DEV), torch.full((1, N), float("nan"), device=DEV)
+    F().gemv_bf16(w, x, out, "f32")
+    assert torch.allclose(out.double(), x.double() @ w.double().T, atol=1e-4, rtol=1e-4)       # as above
+    for row in (0, 7):
+        F().gemv_bf16(w, x[row:row + 1], alone, "f32")
+        assert torch.equal(alone[0], out[row])
+
+
 @pytest.mark.parametrize("M,inter,K", [(1, 256, 128), (4, 12288, 4096), (3, 300, 104), (8, 1000, 512), (8, 640, 5120)])
 def test_gemv_bf16_gate(M, inter, K):
     """silu(gate) * up in the epilogue, over the stacked operand the feed-forward keeps (blocks of 128 gate

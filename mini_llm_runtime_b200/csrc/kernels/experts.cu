@@ -55,18 +55,23 @@ __device__ __forceinline__ int warp_argmax(const float* values, int n) {
     return at == INT_MAX ? 0 : at;
 }
 
+constexpr int kRoutePrefetchRows = 64;    // with more blocks the matrix is on its way anyway (300 rows of 2048 and 128 outputs: 46 us, with it and an early next launch 60 us)
+
 // ROWS tokens a block: the router's matrix is read once for them; then warp r chooses for the block's token r.
-template <typename T, int ROWS>
+// AHEAD: 16-byte pieces of an expert's row that a lane has on their way; eight in steps of few rows, four beyond (150 to 591 rows: 300 of 4096
+// and 64 outputs 45 us, with eight 50 us).
+template <typename T, int ROWS, int AHEAD>
 __global__ void __launch_bounds__(kRouteThreads) route_kernel(const T* x, long long ld, const float* router, const float* correction,
                                                               int rows, int width, int experts, int routed, int groups, int keep, int top,
                                                               int has_gate, int* chosen, float* weights, int* place, int* counts, float* shared_gate,
                                                               float* identity, int kind) {
-    mlr_grid_dependents_may_start();
-    if (ROWS == 1) {
-        // A step of few rows: its router has left the cache since the step before.  It is on its way before the wait.
+    if (ROWS == 1 && gridDim.x <= static_cast<unsigned>(kRoutePrefetchRows)) {
+        // A step of few rows: its router has left the cache since the step before.  It is on its way before the wait, a share by every block; the next launch may start.
+        mlr_grid_dependents_may_start();
         const char* matrix = reinterpret_cast<const char*>(router);
         const size_t bytes = static_cast<size_t>(experts + has_gate) * width * sizeof(float);
-        for (size_t at = threadIdx.x * 128; at < bytes; at += blockDim.x * 128) asm volatile("prefetch.global.L2 [%0];\n" ::"l"(matrix + at));
+        for (size_t at = (static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x) * 128; at < bytes; at += static_cast<size_t>(gridDim.x) * blockDim.x * 128)
+            asm volatile("prefetch.global.L2 [%0];\n" ::"l"(matrix + at));
     }
     mlr_grid_wait();
     extern __shared__ __align__(16) float shared[];
@@ -99,7 +104,7 @@ __global__ void __launch_bounds__(kRouteThreads) route_kernel(const T* x, long l
         float sums[kBoth][ROWS] = {};
         if (width % 4 == 0) {         // 16 bytes at a time (rows of the router and the shared rows start on 16-byte borders then)
             const float4* x4 = reinterpret_cast<const float4*>(xs);
-#pragma unroll ROWS == 1 ? 8 : 4
+#pragma unroll AHEAD
             for (int c = lane; c < width / 4; c += 32) {
                 float4 a[kBoth];
 #pragma unroll
@@ -703,18 +708,20 @@ MLR_API int mlr_experts_route(const void* x, long long ld, int act_bf16, const f
     const int per_block = rows >= 4 * 148 && 4 * one <= 100 * 1024 ? 4 : 1;
     const size_t shared = per_block * one;
     const int threads = rows <= 64 ? kRouteThreads : 256;
-#define MLR_ROUTE(T, ROWS)                                                                                                             \
+#define MLR_ROUTE(T, ROWS, AHEAD)                                                                                                             \
     do {                                                                                                                               \
-        if (shared > 48 * 1024) cudaFuncSetAttribute(route_kernel<T, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(shared)); \
-        mlr_launch((route_kernel<T, ROWS>), dim3((rows + ROWS - 1) / ROWS), dim3(threads), shared, stream, static_cast<const T*>(x), ld, router, \
+        if (shared > 48 * 1024) cudaFuncSetAttribute(route_kernel<T, ROWS, AHEAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(shared)); \
+        mlr_launch((route_kernel<T, ROWS, AHEAD>), dim3((rows + ROWS - 1) / ROWS), dim3(threads), shared, stream, static_cast<const T*>(x), ld, router, \
                    correction, rows, width, experts, routed, groups, keep, top, has_gate, chosen, weights, place, counts, shared_gate, identity, kind); \
     } while (0)
     if (act_bf16) {
-        if (per_block == 4) MLR_ROUTE(__nv_bfloat16, 4);
-        else MLR_ROUTE(__nv_bfloat16, 1);
+        if (per_block == 4) MLR_ROUTE(__nv_bfloat16, 4, 4);
+        else if (rows > kRoutePrefetchRows) MLR_ROUTE(__nv_bfloat16, 1, 4);
+        else MLR_ROUTE(__nv_bfloat16, 1, 8);
     } else {
-        if (per_block == 4) MLR_ROUTE(float, 4);
-        else MLR_ROUTE(float, 1);
+        if (per_block == 4) MLR_ROUTE(float, 4, 4);
+        else if (rows > kRoutePrefetchRows) MLR_ROUTE(float, 1, 4);
+        else MLR_ROUTE(float, 1, 8);
     }
 #undef MLR_ROUTE
     return mlr_launched("experts_route");

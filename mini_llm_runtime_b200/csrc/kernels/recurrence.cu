@@ -1202,12 +1202,13 @@ WalkShape walk_shape(const RecurrenceSpec& s, int n_segments, int rows) {
     w.two = s.rule == 2 && w.fixed_size && columns > 1 && static_cast<long long>(n_segments) * s.heads * columns > mlr_sm_count();
     w.block_cols = kScanBlockCols * (w.two ? 2 : 1);
     w.column_blocks = (s.vdim + w.block_cols - 1) / w.block_cols;
-    // Pieces where whole segments leave the SMs short of blocks: up to eight blocks an SM, and at least six pieces (the two passes take
-    // the time of two pieces, and pieces slow one another).  Measured at 2048 rows of 128 x 128: 64 blocks in 16 pieces 270 -> 150 us,
-    // 128 blocks (two requests) in 9 pieces 281 -> 235 us; 256 blocks in 4 pieces 433 -> 580 us.
+    // Pieces where whole segments leave the SMs short of blocks: room for at least twelve pieces at eight blocks an SM, and segments of at least six
+    // (the two passes take the time of two pieces, and pieces slow one another).  Measured: 64 blocks, 2048 rows of 128 x 128 272 -> 172 us, 800 rows 112 ->
+    // 88 us; 32 blocks, channel decays, 2048 rows 318 -> 144 us.  From 128 blocks on it depends on the lengths: 800 rows of 16 heads 118 -> 144 us, with
+    // channel decays 142 -> 192 us and 2048 rows 348 -> 426 us, two of 900 rows of 8 heads 131 -> 147 us, 2000 and 769 rows 273 -> 223 us.
     const long long blocks = static_cast<long long>(n_segments) * s.heads * w.column_blocks;
     const long long most = std::min(std::min(8ll * mlr_sm_count() / blocks, static_cast<long long>(rows / n_segments / kLeastPiece)), 16ll);
-    w.pieces = s.rule != 1 && w.fixed_size && most >= 6 ? static_cast<int>(most) : 1;
+    w.pieces = s.rule != 1 && w.fixed_size && most >= 6 && 12 * blocks <= 8ll * mlr_sm_count() ? static_cast<int>(most) : 1;
     return w;
 }
 
@@ -1216,7 +1217,7 @@ WalkShape walk_shape(const RecurrenceSpec& s, int n_segments, int rows) {
 // The most ends of pieces a step of up to `rows` rows leaves (0: none is walked in pieces): places of heads * (vdim + 1) * dim values.
 MLR_API int mlr_linear_recurrence_places(const RecurrenceSpec* spec, int rows) {
     int most = 0;
-    for (int n = 1; n <= rows / (6 * kLeastPiece) && n <= 8 * mlr_sm_count() / 6; ++n) {
+    for (int n = 1; n <= rows / (6 * kLeastPiece) && n <= 8 * mlr_sm_count() / 12; ++n) {
         const int pieces = walk_shape(*spec, n, rows).pieces;
         if (pieces > 1) most = std::max(most, n * pieces);
     }

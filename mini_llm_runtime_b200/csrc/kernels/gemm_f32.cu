@@ -18,6 +18,7 @@
 // each from different banks.
 #include "common.cuh"
 
+#include <algorithm>
 #include <climits>
 
 namespace {
@@ -43,11 +44,13 @@ __device__ __forceinline__ void stages_left() { asm volatile("cp.async.wait_grou
 // ---- a tile of BM x BN outputs a block, TM x TN of them a thread (rows and columns dealt round the block) ----
 // Shared memory hands a warp 32 registers a cycle, however few addresses they come from, and the SM's schedulers issue four
 // multiply-adds a warp in that cycle: a thread's TM + TN values of a k for TM * TN multiply-adds bind all tiles but the largest.
-template <int BM, int BN, int TM, int TN, int STAGES, int KK = 32>
+// START, RATE, ROUND: what the tile measured, see tile_cost.
+template <int BM, int BN, int TM, int TN, int STAGES, int KK, int START, int RATE, int ROUND>
 struct Tile {
     static constexpr int kRows = BM, kColumns = BN, kThreadRows = TM, kThreadColumns = TN;
     static constexpr int kThreads = (BM / TM) * (BN / TN);
     static constexpr int kStages = STAGES, kK = KK, kLd = kK + 4;
+    static constexpr int kStart = START, kRate = RATE, kRound = ROUND;
     static constexpr size_t kShared = sizeof(float) * kStages * (BM + BN) * kLd;
 };
 
@@ -215,21 +218,20 @@ int launch_few(const Product& p) {
     return 0;
 }
 
-// What a tile costs a value of K, in cycles of the busiest SM: the registers its warps read from shared memory (1.4 cycles each as
-// measured), or, with few warps, one warp's own way through reads, multiply-adds and its share of the staging.  The constants fit
-// what the tiles measured at 129 rows (6 x 8 a thread: 86 cycles where 78 are computed, 6 x 4: 47 and 48, 4 x 4 in two warps: 57 and 40).
+// What a tile costs a value of K, in cycles, with n blocks on the busiest SM: START + RATE * n, n rounded up to ROUND (2 where blocks run in pairs and a
+// block alone takes a pair's time).  The numbers are fits to every tile at 5 to 2048 rows of ten shapes (1024 x 1024 to 151936 x 1024); by them
+// the choice is within 1 % of the best tile on average, 9 % at worst.  (Computing them from the registers that are read from shared memory missed the
+// largest tile's single round by half: 256 x 4096 x 1024 114 us, with 64 x 64 tiles 66 us.)
 template <typename T>
-double tile_cost(int M, int N) {
+int tile_cost(int M, int N) {
     const long long blocks = ((M + T::kRows - 1LL) / T::kRows) * ((N + T::kColumns - 1LL) / T::kColumns);
-    const double warps = static_cast<double>((blocks + mlr_sm_count() - 1) / mlr_sm_count()) * (T::kThreads / 32);
-    const double reads = 1.4 * warps * (T::kThreadRows + T::kThreadColumns);
-    const double alone = 10.0 + T::kThreadRows + T::kThreadColumns + T::kThreadRows * T::kThreadColumns + 3.0 * (T::kRows + T::kColumns) / T::kThreads;
-    return reads > alone ? reads : alone;
+    const long long busiest = (blocks + mlr_sm_count() - 1) / mlr_sm_count();
+    return static_cast<int>(std::min<long long>(T::kStart + T::kRate * ((busiest + T::kRound - 1) / T::kRound * T::kRound), INT_MAX));
 }
 
 template <bool kVector, typename... Tiles>
 int launch_cheapest(const Product& p) {
-    const double costs[] = {tile_cost<Tiles>(p.M, p.N)...};
+    const int costs[] = {tile_cost<Tiles>(p.M, p.N)...};
     int (*const launches[])(const Product&) = {launch_tile<kVector, Tiles>...};
     int best = 0;
     for (int i = 1; i < static_cast<int>(sizeof...(Tiles)); ++i)
@@ -246,8 +248,10 @@ int choose(const Product& p) {
         if (p.N >= 16 * 2 * mlr_sm_count()) return launch_few<kVector, 16, 16, 1>(p);
         return launch_few<kVector, 8, 16, 1>(p);
     }
-    return launch_cheapest<kVector, Tile<64, 128, 8, 8, 3>, Tile<48, 128, 6, 8, 3>, Tile<32, 128, 4, 8, 3>, Tile<48, 32, 3, 4, 4, 64>,
-                           Tile<16, 64, 2, 4, 4, 64>, Tile<16, 128, 8, 4, 4>, Tile<8, 128, 4, 4, 4>, Tile<16, 32, 2, 2, 5, 64>, Tile<8, 32, 1, 2, 5, 64>>(p);
+    return launch_cheapest<kVector, Tile<64, 128, 8, 8, 3, 32, 10, 100, 2>, Tile<48, 128, 6, 8, 3, 32, 30, 74, 1>, Tile<64, 64, 8, 4, 3, 32, 20, 55, 1>,
+                           Tile<32, 128, 4, 8, 3, 32, 22, 56, 1>, Tile<32, 64, 4, 4, 4, 32, 20, 30, 1>, Tile<48, 32, 3, 4, 4, 64, 15, 26, 1>,
+                           Tile<16, 64, 2, 4, 4, 64, 12, 24, 1>, Tile<16, 128, 8, 4, 4, 32, 2, 41, 2>, Tile<8, 128, 4, 4, 4, 32, 0, 30, 2>,
+                           Tile<16, 32, 2, 2, 5, 64, 10, 13, 1>, Tile<8, 32, 1, 2, 5, 64, 7, 11, 1>>(p);
 }
 
 int product(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw, int ldc, int static_w, cudaStream_t stream) {

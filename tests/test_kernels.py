@@ -180,6 +180,19 @@ def test_gemm_f32_every_tile_gives_the_bits_of_a_row_alone(M, N, K, aligned):
         assert torch.equal(alone[0], out[row]), row
 
 
+@pytest.mark.parametrize("M,N,K,aligned", [(256, 4096, 36, True), (201, 4100, 65, False), (64, 3072, 72, True), (97, 3001, 33, False)])
+def test_gemm_f32_tiles_of_64_columns_give_the_bits_of_a_row_alone(M, N, K, aligned):
+    off = 0 if aligned else 1
+    a, w = torch.randn(M, K + 8, generator=gen(9)).to(DEV)[:, off:off + K], torch.randn(N, K + 8, generator=gen(10)).to(DEV)[:, off:off + K]
+    out, alone = torch.full((M, N), float("nan"), device=DEV), torch.empty(1, N, device=DEV)
+    F().gemm_f32(a, w, out)
+    bound = 2e-7 * math.sqrt(K) * (a.abs().double() @ w.abs().double().T) + 1e-6       # as above
+    assert ((out.double() - a.double() @ w.double().T).abs() <= bound).all()
+    for row in (0, M // 2, M - 1):
+        F().gemm_f32(a[row:row + 1], w, alone)
+        assert torch.equal(alone[0], out[row]), row
+
+
 @pytest.mark.parametrize("M,N,K", [(5, 65535 * 32 + 1, 4), (65535 * 64, 3, 4), (1, 65535 * 64 + 1, 4)])
 def test_gemm_f32_takes_more_tiles_than_a_grid_has_rows(M, N, K):
     a, w = torch.randint(-8, 9, (M, K), generator=gen(7)).float().to(DEV), torch.randint(-8, 9, (N, K), generator=gen(8)).float().to(DEV)

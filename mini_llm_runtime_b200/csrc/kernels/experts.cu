@@ -847,18 +847,18 @@ MLR_API int mlr_experts_product_few(const void* a, long long lda, const int* sou
     int room = 0, device = 0;
     cudaGetDevice(&device);
     cudaDeviceGetAttribute(&room, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
-    room -= 8192 + sums;                        // the kernel's static shared memory and what the driver keeps
-    int slots = room / slot_bytes;
+    room -= 8192;                               // the kernel's static shared memory and what the driver keeps
+    int slots = (room - sums) / slot_bytes;
     if (slots > kFewMostSlots) slots = kFewMostSlots;
     MLR_REQUIRE(slots >= 2, "experts_product: no room for the ring of weights");
     const int bytes = sums + slots * slot_bytes;
     const __nv_bfloat16 *ab = static_cast<const __nv_bfloat16*>(a), *wb = static_cast<const __nv_bfloat16*>(w), *w2b = static_cast<const __nv_bfloat16*>(w2);
     if (gated) {
-        cudaFuncSetAttribute(expert_few_kernel<__nv_bfloat16, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        cudaFuncSetAttribute(expert_few_kernel<__nv_bfloat16, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, room);       // the same at every call: threads may launch side by side
         mlr_launch((expert_few_kernel<__nv_bfloat16, true>), dim3(mlr_sm_count()), dim3(kFewThreads), bytes, stream, ab, lda, source, divisor, wb, w2b,
                    N, K, static_cast<__nv_bfloat16*>(out), ldo, tiles, n_tiles, shape, chunk, slots, status);
     } else {
-        cudaFuncSetAttribute(expert_few_kernel<float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        cudaFuncSetAttribute(expert_few_kernel<float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, room);       // the same at every call: threads may launch side by side
         mlr_launch((expert_few_kernel<float, false>), dim3(mlr_sm_count()), dim3(kFewThreads), bytes, stream, ab, lda, source, divisor, wb, w2b, N, K,
                    static_cast<float*>(out), ldo, tiles, n_tiles, shape, chunk, slots, status);
     }

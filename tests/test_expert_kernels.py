@@ -164,3 +164,35 @@ def test_the_part_takes_rows_off_16_byte_borders(offset):
     x = torch.randn(rows, width + 8, generator=g).bfloat16().cuda()[:, offset:offset + width]
     got, want = part.forward(x, step), part.forward(x.contiguous(), step)
     assert torch.allclose(got, want, atol=1e-2 * float(want.abs().max()), rtol=0)
+
+
+def test_few_rows_of_two_widths_from_two_threads():
+    """The shared memory a launch asks for depends on its K; a thread's smaller launch must not take the limit away under another's larger one."""
+    import threading
+    rows, N = 4, 32
+    status, tiles, n_tiles = torch.zeros(1, dtype=torch.int32, device="cuda"), torch.tensor([0, 0, rows], dtype=torch.int32, device="cuda"), torch.ones(1, dtype=torch.int32, device="cuda")
+    errors, results = [], {}
+
+    def launch(K):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                g = torch.Generator().manual_seed(K)
+                x, w = (torch.randn(n, K, generator=g).bfloat16().cuda() for n in (rows, N))
+                out = torch.empty(rows, N, device="cuda")
+                for _ in range(300):
+                    _call("experts", "mlr_experts_product_few", x.data_ptr(), K, None, 1, w.data_ptr(), None, 0, N, K, out.data_ptr(), N, tiles.data_ptr(),
+                          n_tiles.data_ptr(), rows, 1, 0.0, 0.0, 0.0, status.data_ptr(), _stream())
+                torch.cuda.current_stream().synchronize()
+                results[K] = (out.double(), x.double() @ w.double().T)
+        except Exception as e:
+            errors.append(e)
+
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=launch, args=(K,)) for K in (512, 4096)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors and status.item() == 0
+    for got, want in results.values():
+        assert torch.allclose(got, want, atol=1e-3, rtol=1e-4)         # sums of up to 4096 products of size 1

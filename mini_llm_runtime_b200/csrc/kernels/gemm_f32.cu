@@ -10,9 +10,9 @@
 // and both kernels below give the same bits.
 //
 // Measured (one product, W from memory; before: one kernel of 64 x 64 tiles that waited for every 16 values of K):
-//   2 x 1024 x 3072 (M, N, K): 243 -> 20 us, bound by one thread's chain of multiply-adds; 2 x 151936 x 1024: 574 -> 100 us, 6.2 TB/s;
+//   2 x 1024 x 3072 (M, N, K): 243 -> 22 us, bound by one thread's chain of multiply-adds; 2 x 151936 x 1024: 574 -> 100 us, 6.2 TB/s;
 //   129 x 1024 x 3072: 225 -> 55 us and 129 x 4096 x 1024: 164 -> 46 us, a few warps an SM, bound by their reads of shared memory;
-//   2048 x 4096 x 4096: 1970 -> 1663 us, 41 TFLOP/s, bound by shared memory.
+//   2048 x 4096 x 4096: 1970 -> 1620 us, 42 TFLOP/s, bound by shared memory.
 // Both stage rows of A and W as they lie in memory (asynchronous copies, several stages of K in
 // flight) with their stride padded by 16 bytes, so that 8 neighbouring rows read 4 values of K
 // each from different banks.
@@ -201,12 +201,25 @@ struct Product {
     cudaStream_t stream;
 };
 
+// Blocks on the busiest SM when a grid is dealt out evenly.
+long long busiest_blocks(long long blocks) { return (blocks + mlr_sm_count() - 1) / mlr_sm_count(); }
+
+// Shared memory of a block of which `each` fit an SM and no more.  Blocks are placed while blocks of the kernel before still hold part of the SMs:
+// a grid that could have an SM each ends up with two or three on some of them (a product of 129 rows of 6144 x 1024 behind its norm: 129 us, 59 us
+// so) unless more do not fit.
+size_t shared_for(long long each) {
+    constexpr long long kSm = 228 * 1024, kMostOfBlock = 227 * 1024, kReserved = 1024;       // what sm_100 has, gives a block, and keeps of each block's
+    return static_cast<size_t>(std::max(0ll, std::min(kMostOfBlock, kSm / each / 128 * 128 - kReserved)));
+}
+
 template <bool kVector, typename T>
 int launch_tile(const Product& p) {
     const long long blocks = ((p.M + T::kRows - 1LL) / T::kRows) * ((p.N + T::kColumns - 1LL) / T::kColumns);
     MLR_REQUIRE(blocks <= INT_MAX, "gemm_f32: M=%d N=%d need more than %d tiles", p.M, p.N, INT_MAX);
-    if (allow_shared(gemm_f32_tile_kernel<kVector, T>, T::kShared)) return 1;
-    mlr_launch((gemm_f32_tile_kernel<kVector, T>), dim3(static_cast<unsigned>(blocks)), dim3(T::kThreads), T::kShared, p.stream, p.A, p.W, p.C, p.M, p.N, p.K, p.lda, p.ldw, p.ldc);
+    const size_t bytes = std::max(T::kShared, shared_for(busiest_blocks(blocks)));
+    if (allow_shared(gemm_f32_tile_kernel<kVector, T>, shared_for(1))) return 1;         // the same limit at every call: threads may launch side by side
+    mlr_launch((gemm_f32_tile_kernel<kVector, T>), dim3(static_cast<unsigned>(blocks)), dim3(T::kThreads), bytes, p.stream, p.A, p.W, p.C, p.M, p.N,
+               p.K, p.lda, p.ldw, p.ldc);
     return 0;
 }
 
@@ -224,8 +237,7 @@ int launch_few(const Product& p) {
 // largest tile's single round by half: 256 x 4096 x 1024 114 us, with 64 x 64 tiles 66 us.)
 template <typename T>
 int tile_cost(int M, int N) {
-    const long long blocks = ((M + T::kRows - 1LL) / T::kRows) * ((N + T::kColumns - 1LL) / T::kColumns);
-    const long long busiest = (blocks + mlr_sm_count() - 1) / mlr_sm_count();
+    const long long busiest = busiest_blocks(((M + T::kRows - 1LL) / T::kRows) * ((N + T::kColumns - 1LL) / T::kColumns));
     return static_cast<int>(std::min<long long>(T::kStart + T::kRate * ((busiest + T::kRound - 1) / T::kRound * T::kRound), INT_MAX));
 }
 

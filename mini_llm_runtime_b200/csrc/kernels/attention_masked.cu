@@ -24,7 +24,8 @@
 // the output are float32 or bfloat16.  Keys that are not visible are never loaded.  That kernel serves
 // the float32 path and sizes the others do not take.  In bfloat16, decoded tokens and short portions go to a kernel whose
 // block holds all query heads of ONE kv head (the heads are the rows of its tensor-core tiles, so a range of keys is read
-// once for the group), and `mlr_attention_masked_tiles` (below) takes the prompt portions in tiles of 64 rows.
+// once for the group), and prompt portions go to `attention_masked_tcgen05.cu` in tiles of 128 rows, or, where it does
+// not take the description (two maps a head, keys of more than 128 values), to `mlr_attention_masked_tiles` (below) in tiles of 64.
 #include "attention_spec.cuh"
 #include "common.cuh"
 #include <type_traits>

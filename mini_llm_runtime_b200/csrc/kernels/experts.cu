@@ -11,8 +11,8 @@
 //             the counts are zero again afterwards.
 //   products  over the rows in the order by expert, a tile of rows of ONE expert per block, the rows of the
 //             first product gathered from the tokens' activations:  act = silu(x Wg_e^T) .* (x Wu_e^T), then
-//             y = act Wd_e^T in float32.  Every output adds its K products in the order k = 0 .. K-1 in float32,
-//             so a token's result does not depend on which other tokens share its tile.
+//             y = act Wd_e^T in float32.  Four kernels, by the precision and the number of rows of the step; each adds an output's K
+//             products in float32 in an order of its own that does not depend on which other tokens share the tile.
 //   combine   out[token] = sum_j weight_j y[row of (token, j)]  (+ shared gate * shared expert's result), j in
 //             the order of the choice.
 // A second kind of router (`kind` 1): z = R x + bias (the `correction` operand), the `top` largest z are chosen (ties to
@@ -491,11 +491,11 @@ __global__ void __launch_bounds__(256) expert_product_mma_kernel(const __nv_bflo
 }
 
 // ---- the same product for steps of up to eight rows: a pass over the chosen experts' weights ----
-// An expert then has at most eight rows, and the product is bound by the reading of its weights.  One warp of a block keeps a ring of
+// An expert then has at most eight rows (unless a token chose it more than once, see the kernel), and the product is bound by the reading of its weights.  One warp of a block keeps a ring of
 // slots filled with the weights of 16 rows (a unit; with DUAL 8 rows of each matrix, whose outputs are gated together) by bulk
 // copies of up to 4 KB, 16 warps multiply: warp w takes values 32 w .. 32 w + 31 of every 512 of K, the expert's rows are the second
 // operand of `mma.sync.m16n8k16` and stay in registers while the block's units are of one expert (a block's units are neighbours).
-// The warps' sums are added in warp order, so a result does not depend on the grid or on what else the step holds.  The tiled
+// The warps' sums are added in warp order, so a result depends neither on the grid nor on the step's other rows while there are at most eight.  The tiled
 // kernel above left most of the memory's rate unused at these sizes (a third of the SMs had no block, a block 28 KB on their way):
 // gate/up and down of one row with 4 of 20 outputs at 2048 x 4096: 77 -> 20 and 38 -> 12 us; of three rows with 4 of 16 at 1024 x 2048: 41 -> 16
 // and 19 -> 12 us.

@@ -97,7 +97,7 @@ class Runtime:
         # beyond; in a 2048-token step of the 8B sizes it saves 4 % of the step).
         self.pair_rows = 1024
         self.pair_everything = False  # every product of 256 rows or more on the two-SM kernel
-        self.tcgen05_attention = True  # prompt portions of 65 rows and more on the tcgen05 attention kernel
+        self.tcgen05_attention = True  # prompt portions on the tcgen05 kernels: masked attention's all, plain attention's where one of the step has more than 64 rows
         # Up to this many rows a product runs on the own kernel (swapped operands, split K, partial
         # sums added by the kernel that reads them).  Measured in the decode step of the 8B sizes:
         # it wins by 5 % at 1 to 4 rows, ties at 8 and loses 3-4 % to the vendor library from 16

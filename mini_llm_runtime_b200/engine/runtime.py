@@ -269,7 +269,7 @@ class Runtime:
     # ---- few rows: a pass over the weights with the neighbouring row-wise work folded in
     def _gemv_fits(self, K: int, adds: bool = False) -> bool:
         """Whether the few-row kernel takes `gemv_rows` rows of K values (a product that adds into the stream or stores
-        float32, `adds`, is cut along K until it does)."""
+        float32, `adds`, is cut along K where it does not)."""
         key = (min(self.gemv_rows, 8), K, adds)
         if key not in self._gemv_fit:
             self._gemv_fit[key] = K % 8 == 0 and (adds or bool(native.module("gemv_bf16").mlr_gemv_bf16_fits(key[0], K)))

@@ -10,8 +10,9 @@
 // small.
 //
 // The walk's products are on the tensor cores, each float32 operand split into three bfloat16 parts (24 bits; the six largest of the nine
-// products), sums in float32; the state itself is decayed and added to in float32 on the CUDA cores.  (A value that is not finite reaches the
-// outputs of its whole chunk, not of the tokens behind it alone; other requests never share a chunk.)
+// products), sums in float32; the state itself is decayed and added to in float32 on the CUDA cores.  A value that is not finite breaks such
+// products (an infinity minus its first part, zeros of B times a later token's value): a block that finds one in its outputs or its end of the
+// state throws them away and walks its columns again token by token, so such values reach what the rules say and nothing else.
 //
 // Measured, both kernels against the walk token by token (B200, states of 128 x 128, one request of 2048 tokens): delta rule, 16 heads 59 + 115
 // instead of 358 us; with decays per channel 93 + 111 instead of 400 us; gated linear attention, 16 heads 48 + 88 instead of 310 us; retention,
@@ -402,6 +403,72 @@ __device__ __forceinline__ void chunk_arrive() { asm volatile("bar.arrive %0, %1
 template <int ID, int THREADS>
 __device__ __forceinline__ void chunk_meet() { asm volatile("bar.sync %0, %1;\n" ::"n"(ID), "n"(THREADS) : "memory"); }
 
+// A block's columns of a segment token by token on the CUDA cores, eight lanes a column, for the values that products of parts cannot take.  `room`: shared
+// memory, whose other uses are over.
+template <typename T, int DIM, int RULE, bool CH, int COLS>
+__device__ __forceinline__ void chunk_walk_by_token(const ChunkBuffers& b, const T* proj, int ld, float* columns, int first, int count, int head, int block_col,
+                                                    const RecurrenceSpec& s, float* room) {
+    constexpr int kLanes = 8, E = DIM / kLanes, kThreads = (DIM / 16 + 4) * 32;
+    static_assert(COLS * kLanes <= kThreads);
+    float *ks = room, *qs = ks + kChunk * DIM, *ds = qs + kChunk * DIM, *vs = ds + kChunk * DIM, *gs = vs + kChunk * COLS;
+    const int tid = threadIdx.x, sub = tid % kLanes, col = tid / kLanes;
+    const size_t qk_ld = static_cast<size_t>(s.qk_heads) * DIM, d_ld = static_cast<size_t>(s.heads) * DIM, o_ld = static_cast<size_t>(s.heads) * s.vdim;
+    const size_t qk_at = static_cast<size_t>(head / (s.heads / s.qk_heads)) * DIM, d_at = static_cast<size_t>(head) * DIM, v_at = head * s.vdim + block_col;
+    const bool mine = col < COLS;
+    float* cells = columns + static_cast<size_t>(mine ? col : 0) * DIM + sub;              // every eighth value of the column
+    float S[E];
+#pragma unroll
+    for (int j = 0; j < E; ++j) S[j] = cells[j * kLanes];
+    for (int base = 0; base < count; base += kChunk) {
+        const int n = min(kChunk, count - base);
+        const size_t row0 = static_cast<size_t>(first) + base;
+        for (int i = tid; i < n * DIM; i += kThreads) {
+            const size_t row = row0 + i / DIM;
+            ks[i] = __ldcg(b.kf + row * qk_ld + qk_at + i % DIM);
+            qs[i] = __ldcg(b.qf + row * qk_ld + qk_at + i % DIM);
+            if constexpr (CH) ds[i] = __ldcg(b.df + row * d_ld + d_at + i % DIM);
+        }
+        for (int i = tid; i < n * COLS; i += kThreads) vs[i] = act_in(mlr_load(proj + (row0 + i / COLS) * ld + s.col_v + v_at, i % COLS), s.in_act);
+        if (tid < n) {
+            const float* gate = b.gates + (row0 + tid) * 2 * s.heads + head;
+            if constexpr (!CH) gs[tid] = RULE == 0 ? s.decay[head] : __ldcg(gate);
+            if constexpr (RULE != 0) gs[kChunk + tid] = __ldcg(gate + s.heads);
+        }
+        __syncthreads();
+        if (mine) {                        // whole warps
+            for (int t = 0; t < n; ++t) {
+                const float *k = ks + t * DIM + sub, *q = qs + t * DIM + sub, *d = ds + t * DIM + sub;
+                const float v = vs[t * COLS + col];
+                float held = 0.0f, o = 0.0f;
+                if constexpr (RULE == 1) {
+#pragma unroll
+                    for (int j = 0; j < E; ++j) {
+                        S[j] *= CH ? d[j * kLanes] : gs[t];
+                        held = fmaf(S[j], k[j * kLanes], held);
+                    }
+#pragma unroll
+                    for (int step = 1; step < kLanes; step *= 2) held += __shfl_xor_sync(0xffffffffu, held, step);
+                }
+                const float write = RULE == 0 ? v : gs[kChunk + t] * (v - held);
+#pragma unroll
+                for (int j = 0; j < E; ++j) {
+                    if constexpr (RULE == 1) S[j] = fmaf(k[j * kLanes], write, S[j]);
+                    else S[j] = fmaf(CH ? d[j * kLanes] : gs[t], S[j], k[j * kLanes] * write);
+                    o = fmaf(S[j], q[j * kLanes], o);
+                }
+#pragma unroll
+                for (int step = 1; step < kLanes; step *= 2) o += __shfl_xor_sync(0xffffffffu, o, step);
+                if (RULE == 2) o = fmaf(s.skip[head], v, o);
+                if (sub == 0) b.obuf[(row0 + t) * o_ld + v_at + col] = o;
+            }
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int j = 0; j < E; ++j)
+        if (mine) cells[j * kLanes] = S[j];
+}
+
 // A block walks a segment for 16 * NC columns of a head's state.  Warp w of the first ones keeps the values 16 w .. 16 w + 15 of every column, as
 // the accumulators of a product with the state's columns as its rows: they are the first operand of the products S^T W^T and S^T Q^T as they are.
 // The slices' sums meet in shared memory: two more warps add up the first and make U^T of it, the first operand of what is added to the state,
@@ -424,9 +491,11 @@ __global__ void __launch_bounds__((DIM / 16 + 4) * 32) chunk_walk_kernel(ChunkBu
     if (count <= 0) return;
     const size_t place0 = first / kChunk + segment;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+    bool broken = false;                   // a result of this thread is not finite
     const size_t d_ld = static_cast<size_t>(s.heads) * DIM, o_ld = static_cast<size_t>(s.heads) * s.vdim;
     const size_t ends_ld = CH ? d_ld : static_cast<size_t>(s.heads) * kChunkEnds;
     const float* ends0 = b.ends + place0 * ends_ld + static_cast<size_t>(head) * (CH ? DIM : kChunkEnds);
+    float* columns = state + static_cast<size_t>(slot) * state_stride + (static_cast<size_t>(head) * s.vdim + block_col) * DIM;
     auto wait_stage = [] {
         asm volatile("cp.async.wait_group %0;\n" ::"n"(Stage::kStages - 2) : "memory");
         __syncwarp();
@@ -472,7 +541,7 @@ __global__ void __launch_bounds__((DIM / 16 + 4) * 32) chunk_walk_kernel(ChunkBu
             enext += ends_ld;
         };
         float S[NC][2][4];                 // [column tile][j][(g, 4t + j), (g, 4t + 2 + j), (g + 8, ..), (g + 8, ..)]
-        float* my_state = state + static_cast<size_t>(slot) * state_stride + (static_cast<size_t>(head) * s.vdim + block_col + g) * DIM + warp * 16 + 4 * t;
+        float* my_state = columns + g * DIM + warp * 16 + 4 * t;
 #pragma unroll
         for (int m = 0; m < NC; ++m)
 #pragma unroll
@@ -546,11 +615,16 @@ __global__ void __launch_bounds__((DIM / 16 + 4) * 32) chunk_walk_kernel(ChunkBu
                     }
         });
 #pragma unroll
-        for (int m = 0; m < NC; ++m)
+        for (int i = 0; i < NC * 8; ++i) broken |= !isfinite((&S[0][0][0])[i]);
+        broken = __syncthreads_or(broken);
+        if (!broken) {
 #pragma unroll
-            for (int j = 0; j < 2; ++j)
+            for (int m = 0; m < NC; ++m)
 #pragma unroll
-                for (int i = 0; i < 4; ++i) my_state[(m * 16 + (i >> 1) * 8) * DIM + (i & 1) * 2 + j] = S[m][j][i];
+                for (int j = 0; j < 2; ++j)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) my_state[(m * 16 + (i >> 1) * 8) * DIM + (i & 1) * 2 + j] = S[m][j][i];
+        }
     } else {
         const int nt = warp & 1;           // tokens 8 nt .. 8 nt + 7 (kSlices is even)
         // The slices' sums of a tile, added up.
@@ -671,6 +745,8 @@ __global__ void __launch_bounds__((DIM / 16 + 4) * 32) chunk_walk_kernel(ChunkBu
 #pragma unroll
                         for (int i = 0; i < 4; ++i) o[i] = fmaf(skip, act_in(mlr_load(v, (i & 1) * Stage::kVStride + (i >> 1) * 8), s.in_act), o[i]);
                     }
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) broken |= !isfinite(o[i]);
                     float* to = outputs + m * 16;
                     if (nt * 8 + 2 * t < rows) {
                         to[0] = o[0];
@@ -684,6 +760,11 @@ __global__ void __launch_bounds__((DIM / 16 + 4) * 32) chunk_walk_kernel(ChunkBu
                 outputs += kChunk * o_ld;
             });
         }
+        broken = __syncthreads_or(broken);
+    }
+    if (broken) {
+        static_assert(kChunk * (3 * DIM + Stage::kCols + 2) <= Stage::floats);
+        chunk_walk_by_token<T, DIM, RULE, CH, Stage::kCols>(b, proj, ld, columns, first, count, head, block_col, s, chunk_smem);
     }
     mlr_grid_dependents_may_start();
 }

@@ -129,3 +129,36 @@ def test_chunks_give_what_the_rules_say(rule, dim, vdim, heads, group, segments,
     assert distance(got, want) < 5e-6
     assert distance(state[:, :size].reshape(want_state.shape), want_state) < 5e-6
     assert torch.equal(state[:, size:], c["start"][:, size:])
+
+
+def same_kinds(got, want):
+    """Whether two tensors have NaN, infinities of each sign and finite numbers at the same places."""
+    kind = lambda x: torch.where(torch.isnan(x), 2, torch.where(torch.isinf(x), torch.sign(x), 0)).to(torch.int8)
+    return torch.equal(kind(got), kind(want))
+
+
+@pytest.mark.parametrize("rule", list(RULES))
+@pytest.mark.parametrize("dim,vdim,heads", [(64, 32, 2), (128, 64, 80)])       # one and two column tiles a block
+@pytest.mark.parametrize("where,value", [("v", "nan"), ("v", "inf"), ("k", "nan"), ("k", "inf"), ("q", "nan"), ("state", "nan"), ("state", "inf")])
+def test_a_value_that_is_not_finite_reaches_what_the_rules_say(rule, dim, vdim, heads, where, value):
+    """In the middle of a request's second chunk: the tokens before it, other columns (where the rule keeps them apart) and other requests stay what
+    they are, infinities stay infinities."""
+    c = make(rule, dim, vdim, heads, 1, [40, 20])
+    clean, _, _ = launch(c, c["start"].clone())
+    if where == "state":
+        c["start"][1, 5 * dim + 3] = float(value)              # the first request's column 5 of its first head
+    else:
+        s = c["spec"]
+        c["proj"][24, {"v": s.col_v, "k": s.col_k, "q": s.col_q}[where] + 5] = float(value)
+    state = c["start"].clone()
+    got, _, _ = launch(c, state)
+    want, want_state = exact(c)
+    size = heads * vdim * dim
+    for ours, true in ((got, want), (state[:, :size].reshape(want_state.shape), want_state)):
+        assert same_kinds(ours, true)
+        finite = torch.isfinite(true)
+        assert distance(ours[finite], true[finite]) < 5e-6
+    assert not torch.isfinite(got).all() and torch.isfinite(got[:24] if where != "state" else got[40:]).all()
+    assert torch.equal(got[40:], clean[40:]) and torch.equal(got[:, vdim:], clean[:, vdim:])       # the other request, the other heads
+    if where in ("v", "state"):
+        assert torch.equal(got[:, 32:vdim], clean[:, 32:vdim])             # columns of other blocks

@@ -1361,13 +1361,27 @@ void launch_chunk_walk(const RecurrenceSpec& s, const ChunkBuffers& b, const __n
     mlr_launch(kernel, grid, dim3(ChunkStage<DIM, RULE, CH, NC>::kWarps * 32), shared, stream, b, proj, ld, state, state_stride, segment_info, s);
 }
 
+// Heads that share q and k a block of the preparation: one after the other, so that A and B are made of q and k once, but no more than leave three
+// blocks an SM.  All that share them in one block left the SMs idle: the step rule, 64 heads of 128 x 64 of one q and k, two requests of 80 tokens
+// 97.6 -> 35.0 us (token by token 31.3), 256 tokens 106 -> 42 us (71), 700 tokens 136 -> 75 us (174), 2048 tokens 239 -> 188 us (499); more than 16 give
+// nothing (128 heads, 2048 tokens 363 us with 16, 366 us with 8, 472 us with all).
+int chunk_heads_a_block(const RecurrenceSpec& s, int rows, int n_segments) {
+    if (s.rule == 1 || s.channel_decay) return 1;
+    const int group = s.heads / s.qk_heads;
+    const long long blocks = static_cast<long long>(chunk_places(rows, n_segments)) * s.heads;
+    int most = 1;
+    for (int n = 2; n <= std::min(group, 16); ++n)
+        if (group % n == 0 && blocks / n >= 3ll * mlr_sm_count()) most = n;
+    return most;
+}
+
 template <int DIM, int RULE, bool CH>
 void launch_chunks(const RecurrenceSpec& s, const ChunkBuffers& b, const __nv_bfloat16* proj, int ld, float* state, long long state_stride,
                    const int* segment_info, int n_segments, int rows, cudaStream_t stream) {
     const auto prepare = chunk_prepare_kernel<__nv_bfloat16, DIM, RULE, CH>;
     constexpr size_t shared = chunk_prepare_shared<DIM, CH>();
     if (shared > 48 * 1024) cudaFuncSetAttribute(prepare, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(shared));
-    const int heads_a_block = RULE == 1 || CH ? 1 : s.heads / s.qk_heads;
+    const int heads_a_block = chunk_heads_a_block(s, rows, n_segments);
     mlr_launch(prepare, dim3(chunk_places(rows, n_segments), s.heads / heads_a_block), dim3(kChunkPrepareThreads), shared, stream, b, proj, ld, segment_info,
                n_segments, s, heads_a_block);
     const long long tiles = static_cast<long long>(n_segments) * s.heads * (s.vdim / 16);
@@ -1382,6 +1396,9 @@ void launch_chunks(const RecurrenceSpec& s, const ChunkBuffers& b, const __nv_bf
 MLR_API int mlr_linear_recurrence_in_chunks(const RecurrenceSpec* spec) {
     return spec && (spec->dim == 64 || spec->dim == 128) && spec->vdim % 16 == 0 && spec->vdim >= 16 && !(spec->rule == 2 && spec->channel_decay);
 }
+
+// Heads a block of the chunks' preparation has in a step of `rows` rows in `n_segments` portions.
+MLR_API int mlr_linear_recurrence_chunk_heads(const RecurrenceSpec* spec, int rows, int n_segments) { return chunk_heads_a_block(*spec, rows, n_segments); }
 
 // The three-kernel form with the walk sixteen tokens at a time, for bfloat16 activations.  Arguments as in `mlr_linear_recurrence_pieces`;
 // w (the delta rule; else null), q, k: room of 4 bytes [places, heads * dim * 24] (q, k: qk_heads instead of heads without decays per channel) with

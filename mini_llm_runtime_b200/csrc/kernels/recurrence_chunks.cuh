@@ -137,7 +137,7 @@ __device__ __forceinline__ void chunk_apply(const float (*m)[kChunk + 4], const 
 template <int DIM, bool CH>
 constexpr size_t chunk_prepare_shared() { return sizeof(float) * (DIM + 4) * (CH ? 104 : 48); }
 
-// One block a chunk and `heads_a_block` heads that share q and k (one with decays per channel).  A thread has a pair of tokens for A and B; then the
+// One block a chunk and `heads_a_block` heads that share q and k (one with the delta rule and with decays per channel).  A thread has a pair of tokens for A and B; then the
 // threads of the first half have a value of k each, those of the second a column of V, whose loads have been on their way since the start.
 template <typename T, int DIM, int RULE, bool CH>
 __global__ void __launch_bounds__(kChunkPrepareThreads, RULE == 1 ? 2 : CH ? 3 : 4) chunk_prepare_kernel(ChunkBuffers b, const T* proj, int ld, const int* segment_info,

@@ -162,3 +162,19 @@ def test_a_value_that_is_not_finite_reaches_what_the_rules_say(rule, dim, vdim, 
     assert torch.equal(got[40:], clean[40:]) and torch.equal(got[:, vdim:], clean[:, vdim:])       # the other request, the other heads
     if where in ("v", "state"):
         assert torch.equal(got[:, 32:vdim], clean[:, 32:vdim])             # columns of other blocks
+
+
+@pytest.mark.parametrize("rule,heads,group,segments,most", [("step", 64, 64, [80, 80], 1), ("step", 64, 64, [256], 2), ("step", 64, 64, [2048], 16), ("step", 128, 128, [700], 8),
+                                                            ("decay", 16, 4, [700], 1), ("decay", 16, 4, [2048], 4), ("decay", 48, 3, [2048], 3), ("gla", 64, 64, [2048], 1),
+                                                            ("delta", 64, 64, [2048], 1)])
+def test_heads_a_block_of_the_preparation(rule, heads, group, segments, most):
+    """As many of the heads that share q and k as leave each SM its blocks (148 SMs); q and k of a group are made once whatever it is."""
+    from mini_llm_runtime_b200.ops import native
+    c = make(rule, 128, 16, heads, group, segments)
+    s = c["spec"]
+    a_block = native.module("recurrence").mlr_linear_recurrence_chunk_heads(ctypes.addressof(s), sum(segments), len(segments))
+    assert a_block == most and group % a_block == 0
+    state, (want, want_state) = c["start"].clone(), exact(c)
+    got, _, _ = launch(c, state)
+    assert distance(got, want) < 5e-6
+    assert distance(state[:, :heads * 16 * 128].reshape(want_state.shape), want_state) < 5e-6

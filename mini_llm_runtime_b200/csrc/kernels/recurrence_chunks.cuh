@@ -404,30 +404,38 @@ template <int ID, int THREADS>
 __device__ __forceinline__ void chunk_meet() { asm volatile("bar.sync %0, %1;\n" ::"n"(ID), "n"(THREADS) : "memory"); }
 
 // A block's columns of a segment token by token on the CUDA cores, eight lanes a column, for the values that products of parts cannot take.  `room`: shared
-// memory, whose other uses are over.
+// memory, whose other uses are over.  It is rare, and the walk in chunks must not pay for it: the state is in shared memory and the block's place is asked
+// for anew, since with the state in registers the step rule's walk took 92 registers instead of 80, one block an SM instead of two (1999 tokens of 128
+// heads 325 -> 367 us; so 330 us, the other rules' walks within 3 % of those without it).  2048 tokens of 16 heads, all columns: 2.0 ms.
+template <int DIM, int COLS>
+__host__ __device__ constexpr int by_token_floats() { return kChunk * (3 * DIM + COLS + 2) + COLS * (DIM + 8); }
 template <typename T, int DIM, int RULE, bool CH, int COLS>
-__device__ __forceinline__ void chunk_walk_by_token(const ChunkBuffers& b, const T* proj, int ld, float* columns, int first, int count, int head, int block_col,
+__device__ __forceinline__ void chunk_walk_by_token(const ChunkBuffers& b, const T* proj, int ld, float* state, long long state_stride, const int* segment_info,
                                                     const RecurrenceSpec& s, float* room) {
-    constexpr int kLanes = 8, E = DIM / kLanes, kThreads = (DIM / 16 + 4) * 32;
+    constexpr int kLanes = 8, kThreads = (DIM / 16 + 4) * 32, LD = DIM + 8;                // LD: a warp's four columns fall into different banks
     static_assert(COLS * kLanes <= kThreads);
-    float *ks = room, *qs = ks + kChunk * DIM, *ds = qs + kChunk * DIM, *vs = ds + kChunk * DIM, *gs = vs + kChunk * COLS;
+    float *ks = room, *qs = ks + kChunk * DIM, *ds = qs + kChunk * DIM, *vs = ds + kChunk * DIM, *gs = vs + kChunk * COLS, *S = gs + 2 * kChunk;
     const int tid = threadIdx.x, sub = tid % kLanes, col = tid / kLanes;
+    // Asked for anew: nothing is kept for this through the walk in chunks.
+    const volatile int* info = segment_info + 4 * blockIdx.x;
+    const int first = info[0], count = info[1], slot = info[3], head = blockIdx.y, block_col = blockIdx.z * COLS;
+    float* columns = state + static_cast<size_t>(slot) * state_stride + (static_cast<size_t>(head) * s.vdim + block_col) * DIM;
     const size_t qk_ld = static_cast<size_t>(s.qk_heads) * DIM, d_ld = static_cast<size_t>(s.heads) * DIM, o_ld = static_cast<size_t>(s.heads) * s.vdim;
     const size_t qk_at = static_cast<size_t>(head / (s.heads / s.qk_heads)) * DIM, d_at = static_cast<size_t>(head) * DIM, v_at = head * s.vdim + block_col;
-    const bool mine = col < COLS;
-    float* cells = columns + static_cast<size_t>(mine ? col : 0) * DIM + sub;              // every eighth value of the column
-    float S[E];
-#pragma unroll
-    for (int j = 0; j < E; ++j) S[j] = cells[j * kLanes];
+#pragma unroll 1
+    for (int i = tid; i < COLS * DIM; i += kThreads) S[i / DIM * LD + i % DIM] = columns[i];
+#pragma unroll 1
     for (int base = 0; base < count; base += kChunk) {
         const int n = min(kChunk, count - base);
         const size_t row0 = static_cast<size_t>(first) + base;
+#pragma unroll 1
         for (int i = tid; i < n * DIM; i += kThreads) {
             const size_t row = row0 + i / DIM;
             ks[i] = __ldcg(b.kf + row * qk_ld + qk_at + i % DIM);
             qs[i] = __ldcg(b.qf + row * qk_ld + qk_at + i % DIM);
             if constexpr (CH) ds[i] = __ldcg(b.df + row * d_ld + d_at + i % DIM);
         }
+#pragma unroll 1
         for (int i = tid; i < n * COLS; i += kThreads) vs[i] = act_in(mlr_load(proj + (row0 + i / COLS) * ld + s.col_v + v_at, i % COLS), s.in_act);
         if (tid < n) {
             const float* gate = b.gates + (row0 + tid) * 2 * s.heads + head;
@@ -435,26 +443,26 @@ __device__ __forceinline__ void chunk_walk_by_token(const ChunkBuffers& b, const
             if constexpr (RULE != 0) gs[kChunk + tid] = __ldcg(gate + s.heads);
         }
         __syncthreads();
-        if (mine) {                        // whole warps
+        if (col < COLS) {                  // whole warps
+            float* mine = S + col * LD + sub;                  // every eighth value of the column
+#pragma unroll 1
             for (int t = 0; t < n; ++t) {
                 const float *k = ks + t * DIM + sub, *q = qs + t * DIM + sub, *d = ds + t * DIM + sub;
                 const float v = vs[t * COLS + col];
                 float held = 0.0f, o = 0.0f;
                 if constexpr (RULE == 1) {
-#pragma unroll
-                    for (int j = 0; j < E; ++j) {
-                        S[j] *= CH ? d[j * kLanes] : gs[t];
-                        held = fmaf(S[j], k[j * kLanes], held);
-                    }
+#pragma unroll 4
+                    for (int j = 0; j < DIM; j += kLanes) held = fmaf((CH ? d[j] : gs[t]) * mine[j], k[j], held);
 #pragma unroll
                     for (int step = 1; step < kLanes; step *= 2) held += __shfl_xor_sync(0xffffffffu, held, step);
                 }
                 const float write = RULE == 0 ? v : gs[kChunk + t] * (v - held);
-#pragma unroll
-                for (int j = 0; j < E; ++j) {
-                    if constexpr (RULE == 1) S[j] = fmaf(k[j * kLanes], write, S[j]);
-                    else S[j] = fmaf(CH ? d[j * kLanes] : gs[t], S[j], k[j * kLanes] * write);
-                    o = fmaf(S[j], q[j * kLanes], o);
+#pragma unroll 4
+                for (int j = 0; j < DIM; j += kLanes) {
+                    const float decay = CH ? d[j] : gs[t];
+                    const float value = RULE == 1 ? fmaf(k[j], write, decay * mine[j]) : fmaf(decay, mine[j], k[j] * write);
+                    mine[j] = value;
+                    o = fmaf(value, q[j], o);
                 }
 #pragma unroll
                 for (int step = 1; step < kLanes; step *= 2) o += __shfl_xor_sync(0xffffffffu, o, step);
@@ -464,9 +472,8 @@ __device__ __forceinline__ void chunk_walk_by_token(const ChunkBuffers& b, const
         }
         __syncthreads();
     }
-#pragma unroll
-    for (int j = 0; j < E; ++j)
-        if (mine) cells[j * kLanes] = S[j];
+#pragma unroll 1
+    for (int i = tid; i < COLS * DIM; i += kThreads) columns[i] = S[i / DIM * LD + i % DIM];
 }
 
 // A block walks a segment for 16 * NC columns of a head's state.  Warp w of the first ones keeps the values 16 w .. 16 w + 15 of every column, as
@@ -491,11 +498,10 @@ __global__ void __launch_bounds__((DIM / 16 + 4) * 32) chunk_walk_kernel(ChunkBu
     if (count <= 0) return;
     const size_t place0 = first / kChunk + segment;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
-    bool broken = false;                   // a result of this thread is not finite
+    int broken;                            // some result of the block is not finite
     const size_t d_ld = static_cast<size_t>(s.heads) * DIM, o_ld = static_cast<size_t>(s.heads) * s.vdim;
     const size_t ends_ld = CH ? d_ld : static_cast<size_t>(s.heads) * kChunkEnds;
     const float* ends0 = b.ends + place0 * ends_ld + static_cast<size_t>(head) * (CH ? DIM : kChunkEnds);
-    float* columns = state + static_cast<size_t>(slot) * state_stride + (static_cast<size_t>(head) * s.vdim + block_col) * DIM;
     auto wait_stage = [] {
         asm volatile("cp.async.wait_group %0;\n" ::"n"(Stage::kStages - 2) : "memory");
         __syncwarp();
@@ -541,7 +547,7 @@ __global__ void __launch_bounds__((DIM / 16 + 4) * 32) chunk_walk_kernel(ChunkBu
             enext += ends_ld;
         };
         float S[NC][2][4];                 // [column tile][j][(g, 4t + j), (g, 4t + 2 + j), (g + 8, ..), (g + 8, ..)]
-        float* my_state = columns + g * DIM + warp * 16 + 4 * t;
+        float* my_state = state + static_cast<size_t>(slot) * state_stride + (static_cast<size_t>(head) * s.vdim + block_col + g) * DIM + warp * 16 + 4 * t;
 #pragma unroll
         for (int m = 0; m < NC; ++m)
 #pragma unroll
@@ -614,9 +620,10 @@ __global__ void __launch_bounds__((DIM / 16 + 4) * 32) chunk_walk_kernel(ChunkBu
                         S[m][j][i] = fmaf(decay[(i & 1) * 2 + j], S[m][j][i], added);
                     }
         });
+        float finite = 0.0f;               // stays zero while the state is finite
 #pragma unroll
-        for (int i = 0; i < NC * 8; ++i) broken |= !isfinite((&S[0][0][0])[i]);
-        broken = __syncthreads_or(broken);
+        for (int i = 0; i < NC * 8; ++i) finite = fmaf((&S[0][0][0])[i], 0.0f, finite);
+        broken = __syncthreads_or(finite != 0.0f);
         if (!broken) {
 #pragma unroll
             for (int m = 0; m < NC; ++m)
@@ -627,6 +634,7 @@ __global__ void __launch_bounds__((DIM / 16 + 4) * 32) chunk_walk_kernel(ChunkBu
         }
     } else {
         const int nt = warp & 1;           // tokens 8 nt .. 8 nt + 7 (kSlices is even)
+        float finite = 0.0f;               // stays zero while the outputs are finite
         // The slices' sums of a tile, added up.
         auto summed = [&](const float4* sums, int m) {
             const float4* from = sums + (m * 2 + nt) * kSlices * 32 + lane;
@@ -746,7 +754,7 @@ __global__ void __launch_bounds__((DIM / 16 + 4) * 32) chunk_walk_kernel(ChunkBu
                         for (int i = 0; i < 4; ++i) o[i] = fmaf(skip, act_in(mlr_load(v, (i & 1) * Stage::kVStride + (i >> 1) * 8), s.in_act), o[i]);
                     }
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) broken |= !isfinite(o[i]);
+                    for (int i = 0; i < 4; ++i) finite = fmaf(o[i], 0.0f, finite);         // one instruction a value
                     float* to = outputs + m * 16;
                     if (nt * 8 + 2 * t < rows) {
                         to[0] = o[0];
@@ -760,11 +768,11 @@ __global__ void __launch_bounds__((DIM / 16 + 4) * 32) chunk_walk_kernel(ChunkBu
                 outputs += kChunk * o_ld;
             });
         }
-        broken = __syncthreads_or(broken);
+        broken = __syncthreads_or(finite != 0.0f);
     }
     if (broken) {
-        static_assert(kChunk * (3 * DIM + Stage::kCols + 2) <= Stage::floats);
-        chunk_walk_by_token<T, DIM, RULE, CH, Stage::kCols>(b, proj, ld, columns, first, count, head, block_col, s, chunk_smem);
+        static_assert(by_token_floats<DIM, Stage::kCols>() <= Stage::floats);
+        chunk_walk_by_token<T, DIM, RULE, CH, Stage::kCols>(b, proj, ld, state, state_stride, segment_info, s, chunk_smem);
     }
     mlr_grid_dependents_may_start();
 }

@@ -381,7 +381,9 @@ __global__ void __launch_bounds__(kChunkPrepareThreads, RULE == 1 ? 2 : CH ? 3 :
 template <int DIM, int RULE, bool CH, int NC>
 struct ChunkStage {
     static constexpr int kSlices = DIM / 16, kWarps = kSlices + 4, kCols = 16 * NC;
-    static constexpr int kStages = RULE != 1 && NC == 2 ? 2 : 3;                   // two leave room for two blocks an SM
+    // Two leave room for two blocks an SM.  With 128 decays per channel a block has its SM alone, by three stages' room: two long portions' blocks on one SM
+    // slow each other (gated linear attention, 16 heads, portions of 18, 1664 and four of 1: 198 us alone, 270 us side by side; the delta rule, whose registers leave one, has three as well).
+    static constexpr int kStages = RULE != 1 && NC == 2 && !(CH && DIM == 128) ? 2 : 3;
     // a warp with a slice of the state: W, Q, K and the ends
     static constexpr int w = 0, q = w + (RULE == 1 ? kSliceWords : 0), k = q + kSliceWords, ends = k + kSliceWords, slice = ends + (CH ? 16 : 8);
     // a warp that makes U^T of eight tokens: M V in float32 or V in bfloat16, and the weights P_16 / P_t

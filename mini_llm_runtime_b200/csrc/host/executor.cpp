@@ -72,6 +72,7 @@ enum ArgKind : int32_t {
     kPlan = 8,         // aux: attention plan, i: field (PlanField)
     kStream = 9,
     kLogits = 10,      // where this step's logits go
+    kLongest = 11,     // rows of the step's longest portion
 };
 enum PlanField : int64_t {
     kItems = 0, kItemCount = 1, kChunk = 2, kMaxSplits = 3, kScratch = 4, kCounters = 5,
@@ -301,7 +302,7 @@ struct Model {
 };
 
 struct StepVars {
-    int rows = 0, want = 0, segments = 0, table_stride = 0;
+    int rows = 0, want = 0, segments = 0, longest = 0, table_stride = 0;
     const int32_t* meta[6] = {};
     const int32_t* tables[kMaxGroups] = {};
     const int32_t* extra_base = nullptr;        // device address of element 0 of the metadata buffer
@@ -318,6 +319,7 @@ int64_t resolve(const Arg& a, const StepVars& v) {
         case kRows: return v.rows;
         case kWant: return v.want;
         case kSegments: return v.segments;
+        case kLongest: return v.longest;
         case kMeta: return reinterpret_cast<int64_t>(v.meta[a.aux]);
         case kTable: return reinterpret_cast<int64_t>(v.tables[a.aux]);
         case kTableStride: return v.table_stride;
@@ -592,7 +594,7 @@ int mlr_model_add_program(void* handle, int lo, int hi, int want_lo, int want_hi
         for (int k = 0; k < ops[i].n_args; ++k) {
             const Arg& a = ops[i].args[k];
             if ((a.kind == kMeta && (a.aux < 0 || a.aux > 5)) || (a.kind == kTable && (a.aux < 0 || a.aux >= m->n_groups)) ||
-                (a.kind == kPlan && (a.aux < 0 || a.aux >= static_cast<int>(m->plans.size()))) || a.kind < kImm || a.kind > kLogits)
+                (a.kind == kPlan && (a.aux < 0 || a.aux >= static_cast<int>(m->plans.size()))) || a.kind < kImm || a.kind > kLongest)
                 return fail(1, "model_add_program: op %d argument %d refers to something the model does not have", i, k);
         }
     }
@@ -642,7 +644,7 @@ int mlr_model_step(void* handle, int n, const int32_t* slots, const int32_t* cou
     if (n <= 0) return fail(kStepRefused, "a step needs at least one entry");
     // ---- validate; nothing has changed yet
     std::vector<Segment> segments(static_cast<size_t>(n));
-    int rows = 0;
+    int rows = 0, longest = 0;
     bool all_single = true;
     for (int i = 0; i < n; ++i) {
         if (counts[i] <= 0) return fail(kStepRefused, "the entry of slot %d has no tokens", slots[i]);
@@ -657,6 +659,7 @@ int mlr_model_step(void* handle, int n, const int32_t* slots, const int32_t* cou
                 return fail(kStepRefused, "slot %d wants logits at place %d of %d tokens", slots[i], want_places[w], counts[i]);
         segments[i] = {slots[i], start, counts[i], rows};
         rows += counts[i];
+        longest = std::max(longest, counts[i]);
         all_single = all_single && counts[i] == 1;
     }
     const int want = want_offsets[n];
@@ -760,6 +763,7 @@ int mlr_model_step(void* handle, int n, const int32_t* slots, const int32_t* cou
     vars.rows = rows;
     vars.want = want;
     vars.segments = n;
+    vars.longest = longest;
     vars.table_stride = columns;
     for (int k = 0; k < 6; ++k) vars.meta[k] = m.device_meta + offset[k];
     for (int g = 0; g < m.n_groups; ++g) vars.tables[g] = m.device_meta + offset[6 + g];

@@ -1390,6 +1390,34 @@ void launch_chunks(const RecurrenceSpec& s, const ChunkBuffers& b, const __nv_bf
     else launch_chunk_walk<DIM, RULE, CH, 1>(s, b, proj, ld, state, state_stride, segment_info, n_segments, stream);
 }
 
+// What the two walks of a step weigh, about in microseconds on a B200: the walk token by token for a token of the longest portion (a chain), for a row of
+// all heads' columns, for a portion's state; the walk in chunks for a chunk of the longest portion, for preparing a chunk of all heads, for walking a
+// chunk of all columns, and its longer beginning.  "All" are 128 x 16 values of a state an SM.  Fitted to the choice, not to the times.
+struct WalkWeights {
+    double token, row, portion, chunk, prepare, walk, begin;
+};
+WalkWeights walk_weights(const RecurrenceSpec& s) {
+    if (s.rule == 0) return s.channel_decay ? WalkWeights{0.12, 0.135, 0.2, 0.35, 2.7, 0.85, 5.5} : WalkWeights{0.098, 0.12, 0.45, 0.62, 1.8, 0.74, 5.1};
+    if (s.rule == 1) return s.channel_decay ? WalkWeights{0.13, 0.19, 1.26, 1.08, 8.55, 1.22, 4.1} : WalkWeights{0.163, 0.164, 0.2, 0.5, 5.2, 1.48, 6.5};
+    return WalkWeights{0.15, 0.09, 0.5, 1.0, 0.5, 0.95, 6.3};
+}
+
+// Whether a step is walked sixteen tokens at a time.  A chunk of few rows costs what one of sixteen costs: short portions are walked token by token (16 heads
+// of 128 x 128, delta rule, 128 one-token portions 128 us against 306 in chunks, 64 of 16 tokens 148 against 178), long ones in chunks (2048 tokens 386
+// against 203), a long one beside short ones by what weighs more (2000 and 40 x 1 tokens 658 against 370, 100 and 28 x 1 60 against 87).  Over 2281 steps
+// timed both ways (128 to 6000 rows in 1 to 200 portions of equal and mixed lengths, 4 to 128 heads of 64 and 128 x 32 to 128, a fifth of them not used for
+// the weights) the choice is 0.1 to 0.4 % slower than the better walk on average; in 11 of them it is more than 2 % slower than token by token, at most
+// 14 %, where chunks for every step of 128 rows and more took up to 2.5 times as long.
+bool chunks_are_faster(const RecurrenceSpec& s, int n_segments, int rows, int longest) {
+    if (rows < 128 || 4ll * n_segments > rows) return false;
+    const WalkWeights t = walk_weights(s);
+    const double heads = s.heads * (s.dim / 128.0) / mlr_sm_count(), tiles = heads * (s.vdim / 16);
+    const int pieces = walk_shape(s, n_segments, rows).pieces;             // two passes, the first without outputs
+    const double by_token = t.token * (pieces > 1 ? 2.0 * longest / pieces : longest) + (t.row * (pieces > 1 ? 1.6 : 1.0) * rows + t.portion * n_segments) * tiles;
+    const double chunks = (rows + 15.0 * n_segments) / 16;
+    return by_token > 1.05 * (t.begin + t.chunk * longest / 16 + chunks * (t.prepare * heads + t.walk * tiles));
+}
+
 }  // namespace
 
 // Whether `mlr_linear_recurrence_chunks` takes a description (bfloat16 activations; V read 16 bytes at a time, see there).
@@ -1437,4 +1465,26 @@ MLR_API int mlr_linear_recurrence_chunks(const RecurrenceSpec* spec, const void*
 #undef MLR_CHUNKS
     launch_readout(s, obuf, sd, ld_side, static_cast<const float*>(s.gate_rank ? gf : nullptr), static_cast<__nv_bfloat16*>(out), ld_out, rows, stream);
     return mlr_launched("linear_recurrence_chunks");
+}
+
+// Whether `mlr_linear_recurrence_portions` walks a step of `rows` rows in portions of up to `longest` rows sixteen tokens at a time.
+MLR_API int mlr_linear_recurrence_takes_chunks(const RecurrenceSpec* spec, int n_segments, int rows, int longest) {
+    return mlr_linear_recurrence_in_chunks(spec) && n_segments > 0 && chunks_are_faster(*spec, n_segments, rows, longest);
+}
+
+// `mlr_linear_recurrence_chunks` or `mlr_linear_recurrence_pieces`, whichever is faster for the step's portions, the longest of which has `longest` rows.
+// piece_ends: as `ends` of the latter; places: how many places w, q, k and ends have room for (ceil(rows / 16) + rows / 4 always suffice).
+MLR_API int mlr_linear_recurrence_portions(const RecurrenceSpec* spec, const void* proj, int ld, const void* side, int ld_side, void* out, int ld_out,
+                                           float* state, long long state_stride, const int* segment_info, int n_segments, int longest, const int* positions,
+                                           int rows, float* qf, float* kf, float* gates, float* obuf, float* df, float* gf, int products_made,
+                                           float* piece_ends, int places, uint32_t* w, uint32_t* q, uint32_t* k, float* bm, float* ends, cudaStream_t stream) {
+    MLR_REQUIRE(spec, "linear_recurrence_portions: no description");
+    if (check_recurrence(*spec)) return 1;
+    if (!mlr_linear_recurrence_takes_chunks(spec, n_segments, rows, longest))
+        return mlr_linear_recurrence_pieces(spec, proj, ld, side, ld_side, 1, out, ld_out, state, state_stride, segment_info, n_segments, positions, rows, qf,
+                                            kf, gates, obuf, df, gf, products_made, piece_ends, stream);
+    MLR_REQUIRE(chunk_places(rows, n_segments) <= places, "linear_recurrence_portions: %d rows in %d portions do not fit room for %d chunks", rows, n_segments,
+                places);
+    return mlr_linear_recurrence_chunks(spec, proj, ld, side, ld_side, out, ld_out, state, state_stride, segment_info, n_segments, positions, rows, qf, kf,
+                                        gates, obuf, df, gf, products_made, w, q, k, bm, ends, stream);
 }

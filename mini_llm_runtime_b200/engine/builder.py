@@ -35,7 +35,7 @@ PLAN_FIELDS = {"items": 0, "n_items": 1, "chunk": 2, "max_splits": 3, "scratch":
                # derived: the split-KV items when the step has no prompt tiles / when it has some; all prompt tiles
                "n_items_alone": 10, "n_items_beside": 11, "n_prompt_tiles": 12}
 
-K_IMM, K_FLOAT, K_ROWS, K_WANT, K_SEGMENTS, K_META, K_TABLE, K_TABLE_STRIDE, K_PLAN, K_STREAM, K_LOGITS = range(11)
+K_IMM, K_FLOAT, K_ROWS, K_WANT, K_SEGMENTS, K_META, K_TABLE, K_TABLE_STRIDE, K_PLAN, K_STREAM, K_LOGITS, K_LONGEST = range(12)
 NEED_ALWAYS, NEED_WANTED, NEED_PLAN_FIELD = 0, 1, 2
 MAX_ARGS = 30
 
@@ -183,6 +183,11 @@ class EagerBuilder(_NormHints):
     def segments(self) -> int:
         return len(self.step.segments)
 
+    @property
+    def longest(self) -> int:
+        """Rows of the step's longest portion."""
+        return max(s.count for s in self.step.segments)
+
     def plan(self, spec: Tuple[int, int, int, int, int, int]) -> PlanRef:
         """spec: (query heads per kv head, kv heads, window, wide tiles (0 none, 1 where a portion has more than 64 rows, 2 for all), head size, small allowed)."""
         key = ("attention_plan",) + tuple(spec)
@@ -253,6 +258,7 @@ class ProgramBuilder(_NormHints):
         self.status = status_ptr
         self.stream = Sym(K_STREAM)
         self.segments = Sym(K_SEGMENTS)
+        self.longest = Sym(K_LONGEST)
         self.residual: Optional[Buf] = None
         self.ops: List[OpRecord] = []
         self.names: List[str] = []          # the entry point of each op, for whoever wants to read a program

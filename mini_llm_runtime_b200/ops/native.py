@@ -127,6 +127,10 @@ _SIGNATURES = {
                                         c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p],
         "mlr_linear_recurrence_in_chunks": [c_void_p],
         "mlr_linear_recurrence_chunk_heads": [c_void_p, c_int, c_int],
+        "mlr_linear_recurrence_takes_chunks": [c_void_p, c_int, c_int, c_int],
+        "mlr_linear_recurrence_portions": [c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_longlong, c_void_p, c_int, c_int,
+                                           c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p,
+                                           c_void_p, c_void_p, c_void_p, c_void_p, c_void_p],
         "mlr_linear_recurrence_chunks": [c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_longlong, c_void_p, c_int, c_void_p,
                                          c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
                                          c_void_p, c_void_p, c_void_p],

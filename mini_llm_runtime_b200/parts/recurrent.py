@@ -60,23 +60,22 @@ def emit_recurrence(b, mixer, proj, side, act, run: RunContext) -> None:
     gates = b.temp(proj.rows, 2 * d.heads, torch.float32)
     obuf = b.temp(proj.rows, d.heads * d.vdim, torch.float32)
     lib = native.module("recurrence")
-    if proj.is_bf16 and b.ge(proj.rows, 128) and proj.ld % 8 == 0 and d.col_v % 8 == 0 and proj.ptr % 16 == 0 and lib.mlr_linear_recurrence_in_chunks(address(d)):
-        # Sixteen tokens at a time.  Below 128 rows the extra launch costs what the walk saves (16 heads of 128 x 128, delta rule: 70 rows 22 us either
-        # way, 300 rows 86 -> 71 us, 2048 rows 373 -> 195 us).
-        bound = b.bound(proj.rows)
-        places = (bound + 15) // 16 + min(bound, state.shape[0])
+    # Room for the ends of a walk's pieces, where steps of this many rows can be walked in pieces.
+    bound = b.bound(proj.rows)
+    pieces = lib.mlr_linear_recurrence_places(address(d), bound)
+    ends = b.temp(pieces, d.heads * (d.vdim + 1) * d.dim, torch.float32) if pieces else None
+    if proj.is_bf16 and proj.ld % 8 == 0 and d.col_v % 8 == 0 and proj.ptr % 16 == 0 and lib.mlr_linear_recurrence_in_chunks(address(d)):
+        # The entry point chooses between sixteen tokens at a time and one by the step's portions; chunks are for at most a portion to four rows.
+        places = (bound + 15) // 16 + min(bound // 4, state.shape[0])
         operand = lambda heads: b.temp(places, heads * d.dim * 24, torch.float32)
         shared = d.heads if d.channel_decay else d.qk_heads
         w = operand(d.heads) if d.rule == RecurrenceSpec.RULE["delta"] else None
         q, k, bm = operand(shared), operand(shared), b.temp(proj.rows, d.heads * 16, torch.float32)
-        ends = b.temp(places, d.heads * (d.dim if d.channel_decay else 36), torch.float32)
-        b.launch("recurrence", "mlr_linear_recurrence_chunks", address(d), proj.ptr, proj.ld, side.ptr, side.ld, act.ptr, act.ld, state.data_ptr(),
-                 state.stride(0), info, b.segments, b.meta("positions"), proj.rows, qf.ptr, kf.ptr, gates.ptr, obuf.ptr, df.ptr if df else None,
-                 gf.ptr if gf else None, made, w.ptr if w else None, q.ptr, k.ptr, bm.ptr, ends.ptr, b.stream)
+        chunk_ends = b.temp(places, d.heads * (d.dim if d.channel_decay else 36), torch.float32)
+        b.launch("recurrence", "mlr_linear_recurrence_portions", address(d), proj.ptr, proj.ld, side.ptr, side.ld, act.ptr, act.ld, state.data_ptr(),
+                 state.stride(0), info, b.segments, b.longest, b.meta("positions"), proj.rows, qf.ptr, kf.ptr, gates.ptr, obuf.ptr, df.ptr if df else None,
+                 gf.ptr if gf else None, made, ends.ptr if ends else None, places, w.ptr if w else None, q.ptr, k.ptr, bm.ptr, chunk_ends.ptr, b.stream)
         return
-    # Room for the ends of a walk's pieces, where steps of this many rows can be walked in pieces.
-    places = lib.mlr_linear_recurrence_places(address(d), b.bound(proj.rows))
-    ends = b.temp(places, d.heads * (d.vdim + 1) * d.dim, torch.float32) if places else None
     b.launch("recurrence", "mlr_linear_recurrence_pieces", address(d), proj.ptr, proj.ld, side.ptr, side.ld, proj.is_bf16, act.ptr,
              act.ld, state.data_ptr(), state.stride(0), info, b.segments, b.meta("positions"), proj.rows, qf.ptr, kf.ptr, gates.ptr,
              obuf.ptr, df.ptr if df else None, gf.ptr if gf else None, made, ends.ptr if ends else None, b.stream)

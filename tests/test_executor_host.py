@@ -13,7 +13,7 @@ import pytest
 
 from mini_llm_runtime_b200.cache.manager import CacheManager, GroupSpec
 from mini_llm_runtime_b200.engine import executor as X
-from mini_llm_runtime_b200.engine.builder import (K_FLOAT, K_IMM, K_META, K_PLAN, K_ROWS, K_SEGMENTS, K_TABLE, K_TABLE_STRIDE,
+from mini_llm_runtime_b200.engine.builder import (K_FLOAT, K_IMM, K_LONGEST, K_META, K_PLAN, K_ROWS, K_SEGMENTS, K_TABLE, K_TABLE_STRIDE,
                                                   K_WANT, NEED_PLAN_FIELD, NEED_WANTED, OpRecord, PLAN_FIELDS)
 
 PAGE = 4
@@ -125,6 +125,15 @@ def test_a_step_hands_its_launches_what_the_step_knows():
     assert code == X.STEP_OK
     first = host.recorded()[0]
     assert section(host, first[4], 3) == [1, 2, 6] and host.ledger([a, b])[2] == [7, 3]
+
+
+def test_launches_are_handed_the_longest_portion():
+    host = Host()
+    a, b = host.cache.open(), host.cache.open()
+    host.program([host.op([(K_LONGEST, 0, 0), (K_SEGMENTS, 0, 0)] + [(K_IMM, 0, 0)] * 7)])
+    for portions, longest in ([(a, [5], []), (b, [7, 8, 9], [])], 3), ([(b, [1, 2], []), (a, [3], [])], 2), ([(a, [4], [0]), (b, [4], [0])], 1):
+        assert host.step(portions)[0] == X.STEP_OK, host.error()
+        assert host.recorded()[0][:2] == [longest, 2]
 
 
 def test_refusals_before_device_work_change_nothing():

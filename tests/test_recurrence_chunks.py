@@ -178,3 +178,49 @@ def test_heads_a_block_of_the_preparation(rule, heads, group, segments, most):
     got, _, _ = launch(c, state)
     assert distance(got, want) < 5e-6
     assert distance(state[:, :heads * 16 * 128].reshape(want_state.shape), want_state) < 5e-6
+
+
+def launch_portions(c, state, longest):
+    """The outputs of the entry point that chooses the walk; room as a step's description asks for it, with a margin that must stay as it is."""
+    from mini_llm_runtime_b200.ops import native
+    s, proj, rows, n = c["spec"], c["proj"], c["proj"].shape[0], len(c["segments"])
+    f32 = lambda *shape: torch.full(shape, float("nan"), device="cuda")
+    out = torch.empty(rows, s.heads * s.vdim, device="cuda", dtype=torch.bfloat16)
+    q, k, gates, obuf, df = f32(rows, s.qk_heads * s.dim), f32(rows, s.qk_heads * s.dim), f32(rows, 2 * s.heads), f32(rows, s.heads * s.vdim), f32(rows, s.heads * s.dim)
+    pieces = native.module("recurrence").mlr_linear_recurrence_places(ctypes.addressof(s), rows)
+    piece_ends = f32(pieces, s.heads * (s.vdim + 1) * s.dim) if pieces else None
+    places = (rows + 15) // 16 + min(rows // 4, n)
+    held = [f32(places + 1, s.heads * s.dim * 24), f32(places + 1, (s.heads if s.channel_decay else s.qk_heads) * s.dim * 24),
+            f32(places + 1, (s.heads if s.channel_decay else s.qk_heads) * s.dim * 24), f32(rows + 1, s.heads * 16), f32(places + 1, s.heads * (s.dim if s.channel_decay else 36))]
+    native.call("recurrence", "mlr_linear_recurrence_portions", ctypes.addressof(s), proj.data_ptr(), proj.stride(0), proj.data_ptr(), proj.stride(0),
+                out.data_ptr(), out.stride(0), state.data_ptr(), state.stride(0), c["info"].data_ptr(), n, longest, c["positions"].data_ptr(), rows,
+                q.data_ptr(), k.data_ptr(), gates.data_ptr(), obuf.data_ptr(), df.data_ptr(), None, 0, piece_ends.data_ptr() if pieces else None, places,
+                *[t.data_ptr() for t in held], native.stream())
+    torch.cuda.synchronize()
+    assert all(torch.isnan(t[-1]).all() for t in held)
+    return obuf
+
+
+@pytest.mark.parametrize("rule,dim,vdim,heads,segments,chunks", [
+    ("delta", 128, 128, 16, [1] * 128, False), ("delta", 128, 128, 16, [16] * 64, False), ("delta", 128, 128, 16, [100] + [1] * 28, False),
+    ("delta", 128, 128, 16, [2000] + [1] * 40, True), ("delta", 128, 128, 16, [128], True), ("channel_delta", 128, 128, 16, [1] * 256, False),
+    ("channel_delta", 128, 128, 16, [700], True), ("gla", 64, 64, 16, [8] * 32, False), ("gla", 128, 128, 16, [3, 900, 1], True), ("decay", 64, 64, 8, [2048], False),
+    ("decay", 128, 128, 8, [2048], True), ("decay", 128, 128, 8, [1] * 130, False), ("step", 128, 64, 64, [16] * 40, False), ("step", 128, 64, 64, [600], True),
+    ("step", 128, 64, 64, [1] * 128, False), ("step", 128, 64, 64, [127], False),
+])
+def test_the_walk_is_chosen_by_the_portions_of_a_step(rule, dim, vdim, heads, segments, chunks):
+    """Short portions token by token, long ones in chunks (each pair of times beside the rule), in the same bits as the entry points of either walk."""
+    from mini_llm_runtime_b200.ops import native
+    c = make(rule, dim, vdim, heads, heads if rule == "step" else 1, segments)
+    takes = native.module("recurrence").mlr_linear_recurrence_takes_chunks(ctypes.addressof(c["spec"]), len(segments), sum(segments), max(segments))
+    assert bool(takes) == chunks
+    state, alone = c["start"].clone(), c["start"].clone()
+    got = launch_portions(c, state, max(segments))
+    if chunks:
+        want, _, _ = launch(c, alone)
+        assert torch.equal(got, want) and torch.equal(state, alone)
+    elif not native.module("recurrence").mlr_linear_recurrence_places(ctypes.addressof(c["spec"]), sum(segments)):
+        want, _, _ = launch(c, alone, chunks=False)
+        assert torch.equal(got, want) and torch.equal(state, alone)
+    else:
+        assert distance(got, exact(c)[0]) < 5e-6

@@ -71,7 +71,19 @@ SMALL_D = {
     ],
 }
 
-ALL = {"small_a": SMALL_A, "small_b": SMALL_B, "small_c": SMALL_C, "small_d": SMALL_D}
+# States of 64 and 128 keys by a multiple of 16 values: in bfloat16 their long portions are walked sixteen tokens at a time.
+SMALL_E = {
+    "architecture": "Gopevik", "vocab": 90, "width": 64, "norm": {"eps": 1e-6, "groups": 2},
+    "layers": [
+        _parallel({"heads": 2, "kv_heads": 1, "dim": 16, "vdim": 16, "scale": 0.3, "mask": {"size": 40}, "rot": {"base": 100.0, "dims": 16}},
+                  {"heads": 2, "dim": 64, "vdim": 32, "decay": [0.9, 0.99], "rot": {"base": 500.0, "dims": 48}},
+                  0.9, 1.1, 48),
+        _delta(2, 1, 128, 16, 4, 40),
+        _delta(2, 2, 64, 48, 3, None),
+    ],
+}
+
+ALL = {"small_a": SMALL_A, "small_b": SMALL_B, "small_c": SMALL_C, "small_d": SMALL_D, "small_e": SMALL_E}
 
 
 def get(name: str) -> dict:

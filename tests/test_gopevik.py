@@ -493,6 +493,24 @@ def test_whole_prompts_portions_and_decoding_agree_with_the_plain_implementation
 
 
 @pytest.mark.gpu
+def test_long_portions_of_both_mixers_are_walked_in_chunks(case):
+    """The sizes of small_e reach the walk sixteen tokens at a time through the engine; the test above holds its logits."""
+    from mini_llm_runtime_b200.ops import native
+    from mini_llm_runtime_b200.ops.specs import RecurrenceSpec, address
+    folder, config, weights = case
+    if config["vocab"] != gopevik_models.get("small_e")["vocab"]:
+        pytest.skip("states of other sizes")
+    model = engine_model(folder, "bfloat16", num_pages=24, page_size=8, max_requests=2)
+    run_whole(model, tokens_for(config, 150, 4))
+    programs = [names for (lo, hi, *_), names in model._native.programs.items() if lo <= 150 <= hi]
+    assert programs and programs[0].count("mlr_linear_recurrence_portions") == 3
+    lib = native.module("recurrence")
+    for heads, dim, vdim, rule in ((2, 64, 32, "decay"), (2, 128, 16, "delta"), (2, 64, 48, "delta")):
+        spec = RecurrenceSpec(heads=heads, qk_heads=1, dim=dim, vdim=vdim, rule=RecurrenceSpec.RULE[rule])
+        assert lib.mlr_linear_recurrence_takes_chunks(address(spec), 1, 150, 150) and not lib.mlr_linear_recurrence_takes_chunks(address(spec), 75, 150, 2)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 def test_a_batch_of_unequal_requests_equals_each_alone_and_slots_are_used_again(case, dtype):
     from mini_llm_runtime_b200.engine.model import StepEntry

@@ -224,3 +224,75 @@ def test_the_walk_is_chosen_by_the_portions_of_a_step(rule, dim, vdim, heads, se
         assert torch.equal(got, want) and torch.equal(state, alone)
     else:
         assert distance(got, exact(c)[0]) < 5e-6
+
+
+@pytest.mark.parametrize("rule,dim,vdim,heads,group,segments", [
+    ("decay", 128, 128, 2, 1, [2048]), ("gla", 128, 128, 2, 1, [2048]), ("delta", 128, 128, 2, 1, [2048]), ("channel_delta", 128, 128, 2, 1, [2048]),
+    ("step", 128, 64, 2, 2, [1999]), ("delta", 64, 256, 2, 1, [130, 70]), ("channel_delta", 128, 256, 2, 2, [90, 33]), ("delta", 64, 64, 80, 1, [64] * 3),
+    ("step", 64, 48, 3, 3, [5, 17, 1] * 100), ("channel_delta", 64, 16, 2, 1, [1, 2, 30] * 110), ("decay", 64, 32, 2, 1, [7] * 300),
+])
+def test_chunks_are_as_exact_as_the_walk_token_by_token_and_repeat_their_bits(rule, dim, vdim, heads, group, segments):
+    """Long portions, columns past the first 128, more than 256 portions.  Both walks add in float32, in other orders, so their distances from 64 bits are
+    of one size (1e-8 to 3e-7, chunks at most 1.3 times the other's where measured); limit: three times, and 2e-8 for sums of few terms.  A split
+    into two bfloat16 parts instead of three is 16 bits of each operand: 2^-17 of a term, over 4e-6."""
+    c = make(rule, dim, vdim, heads, group, segments)
+    want, want_state = exact(c)
+    size = heads * vdim * dim
+    def run(chunks):
+        state = c["start"].clone()
+        got, _, _ = launch(c, state, chunks=chunks)
+        return got, state[:, :size].reshape(want_state.shape)
+    (got, state), (by_token, by_token_state) = run(True), run(False)
+    assert distance(got, want) < 3 * distance(by_token, want) + 2e-8
+    assert distance(state, want_state) < 3 * distance(by_token_state, want_state) + 2e-8
+    for _ in range(3):
+        again, state_again = run(True)
+        assert torch.equal(again, got) and torch.equal(state_again, state)
+
+
+@pytest.mark.parametrize("rule,rotated,made", [("decay", True, 0), ("gla", False, 1), ("channel_delta", False, 0), ("channel_delta", False, 1)])
+def test_both_walks_give_the_same_read_out(rule, rotated, made):
+    """Rotated q and k, low-rank decays and gates made by the kernel or beforehand, norm, weight and gate: the entry points differ in the walk alone, so
+    their bfloat16 results differ by at most a rounding of values that differ by some 1e-7: one place of eight bits, for few of them."""
+    from mini_llm_runtime_b200.ops import native
+    dim = vdim = 64
+    heads, rank, segments = 2, 16, [70, 100]
+    c = make(rule, dim, vdim, heads, 1, segments)
+    s, proj, rows = c["spec"], c["proj"], sum(segments)
+    g = torch.Generator().manual_seed(5)
+    side = torch.randn(rows, heads * vdim, generator=g).cuda().bfloat16()
+    weight = (1 + 0.1 * torch.randn(vdim, generator=g)).cuda()
+    freq = (100.0 ** (-torch.arange(16) / 16)).cuda()
+    gate_w = (torch.randn(rank, heads * vdim, generator=g) * rank ** -0.5).cuda().bfloat16()
+    if rotated:
+        s.prep, s.rot_dims, s.freq = RecurrenceSpec.PREP["rotate"], 32, freq.data_ptr()
+    s.out_weight, s.gate_kind = weight.data_ptr(), 1
+    wide = torch.cat([proj, side], 1).contiguous()             # the gate's columns behind the projections
+    s.col_gate = proj.shape[1]
+    if s.channel_decay:
+        s.gate_rank, s.gate_w = rank, gate_w.data_ptr()
+    results = []
+    for chunks in (True, False):
+        f32 = lambda *shape: torch.full(shape, float("nan"), device="cuda")
+        out = torch.empty(rows, heads * vdim, device="cuda", dtype=torch.bfloat16)
+        state = c["start"].clone()
+        q, k, gates, obuf, df, gf = f32(rows, heads * dim), f32(rows, heads * dim), f32(rows, 2 * heads), f32(rows, heads * vdim), f32(rows, heads * dim), f32(rows, heads * vdim)
+        if made:
+            df.copy_(wide[:, s.col_a:s.col_a + rank].float() @ c["held"]["decay_w"].float())
+            gf.copy_(wide[:, s.col_gate:s.col_gate + rank].float() @ gate_w.float())
+        common = [ctypes.addressof(s), wide.data_ptr(), wide.stride(0), wide.data_ptr(), wide.stride(0)]
+        tail = [out.data_ptr(), out.stride(0), state.data_ptr(), state.stride(0), c["info"].data_ptr(), len(segments), c["positions"].data_ptr(), rows,
+                q.data_ptr(), k.data_ptr(), gates.data_ptr(), obuf.data_ptr(), df.data_ptr(), gf.data_ptr(), made]
+        places = (rows + 15) // 16 + len(segments)
+        held = [f32(places, heads * dim * 24) for _ in range(3)] + [f32(rows, heads * 16), f32(places, heads * (dim if s.channel_decay else 36))]
+        if chunks:
+            native.call("recurrence", "mlr_linear_recurrence_chunks", *common, *tail, *[t.data_ptr() for t in held], native.stream())
+        else:
+            native.call("recurrence", "mlr_linear_recurrence_split", *common, 1, *tail, native.stream())
+        torch.cuda.synchronize()
+        results.append((out.float(), state))
+    (got, state), (want, want_state) = results
+    assert torch.isfinite(got).all() and float(want.square().mean()) > 0.05
+    off = (got - want).abs() > 1e-6 * want.abs().max()
+    assert float(off.float().mean()) < 1e-3 and bool(((got - want).abs() <= 2.0 ** -7 * want.abs() + 1e-6).all())
+    assert distance(state, want_state.double()) < 1e-6

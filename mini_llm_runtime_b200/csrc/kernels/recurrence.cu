@@ -318,8 +318,8 @@ __global__ void __launch_bounds__(1024) linear_recurrence_kernel(const T* proj, 
 // ---- the same in three kernels, for steps of many rows.  The fused kernel above has one block per (request, head):
 // a long prompt of one request then runs on a handful of SMs, and every block prepares q and k itself.  Here the
 // preparation and the read-out are parallel over rows, and the scan, the only sequential part, has a block per
-// (request, head, group of 16 columns of the state).  In bfloat16, from 128 rows on, states of 64 or 128 by a multiple of 16 are walked sixteen
-// tokens at a time instead (recurrence_chunks.cuh).
+// (request, head, group of 16 columns of the state).  In bfloat16, long portions over states of 64 or 128 by a multiple of 16 are walked sixteen
+// tokens at a time instead (recurrence_chunks.cuh; `chunks_are_faster` says which steps).
 
 // q and k of every row, prepared, as float32 [rows, qk_heads * dim] each; for the delta rule also g and beta, for the step rule g and dt [rows, 2 * heads].  zf
 // (or null): [rows, heads * dim], z of every key channel without its bias, turned into the channel's decay in place.

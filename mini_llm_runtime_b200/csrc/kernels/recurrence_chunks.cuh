@@ -14,12 +14,12 @@
 // products (an infinity minus its first part, zeros of B times a later token's value): a block that finds one in its outputs or its end of the
 // state throws them away and walks its columns again token by token, so such values reach what the rules say and nothing else.
 //
-// Measured, both kernels against the walk token by token (B200, states of 128 x 128, one request of 2048 tokens): delta rule, 16 heads 59 + 115
-// instead of 358 us; with decays per channel 93 + 111 instead of 400 us; gated linear attention, 16 heads 48 + 88 instead of 310 us; retention,
-// 8 heads 13 + 94 instead of 242 us (in pieces 172 us); the step rule, 1999 tokens of 128 heads of 128 x 64, 38 + 231 instead of 470 us.  What a
-// chunk takes, 0.7 to 0.9 us, is the chain from one state to the next: splitting it, a product, the meeting of the warps, a product.  Distance of
-// the outputs from 64 bits over 2048 tokens: 1.4e-7 with the delta rule (token by token 1.3e-7), 1.0e-7 (2.0e-7) retention, 1.7e-7 (1.7e-7)
-// gated linear attention, 2.8e-8 (2.8e-8) step.
+// Measured, both kernels against the walk token by token (B200, states of 128 x 128, one request of 2048 tokens): delta rule, 16 heads 59 + 118
+// instead of 358 us; with decays per channel 90 + 111 instead of 404 us; gated linear attention, 16 heads 50 + 87 instead of 312 us; retention,
+// 8 heads 15 + 95 instead of 242 us (in pieces 173 us); the step rule, 1999 tokens of 128 heads of 128 x 64 in 8 groups, 40 + 241 instead of 475 us.  What a
+// chunk takes, 0.7 to 0.9 us (1.9 us for the step rule's 256 blocks, two an SM), is the chain from one state to the next: splitting it, a product, the
+// meeting of the warps, a product.  Distance of the outputs from 64 bits over 2048 tokens: 1.4e-7 with the delta rule (token by token 1.3e-7), 1.0e-7 (2.0e-7)
+// retention, 1.7e-7 (1.7e-7) gated linear attention, 2.8e-8 (2.8e-8) step; held beside the walk token by token by tests/test_recurrence_chunks.py.
 //
 // Sixteen tokens a chunk are the rows of one instruction.  Two column tiles a block where the tiles outnumber the SMs: what a block reads of W, Q
 // and K serves both.
